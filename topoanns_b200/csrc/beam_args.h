@@ -18,6 +18,11 @@ struct BeamArgs {
     Cand* out_cand;
     uint32_t* out_stats;
     uint32_t* status;
+    // of beam_short_kernel and beam_long_kernel:
+    uint32_t list_len, two_lists;   // long: entries of the list, whether it is double-buffered
+    uint32_t pool_len;              // short: entries of the tail's pool (0 = none)
+    uint32_t only_marked;           // long: search only the queries that beam_short_kernel marked in their statistics
+    const float* pivots_packed;  // PackPivots() of the index's pivots, or nullptr
 };
 
 }  // namespace tann

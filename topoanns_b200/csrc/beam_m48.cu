@@ -1,0 +1,10 @@
+// The beam-search kernels for 48 chunks.
+#include "beam_long.cuh"
+#include "beam_short.cuh"
+
+namespace tann {
+BeamKernelFn PickShort48(uint32_t rounds, int kind, uint32_t list_regs) {
+    return list_regs == 1 ? PickShortOf<48, 1>(rounds, kind) : (list_regs == 2 ? PickShortOf<48, 2>(rounds, kind) : PickShortOf<48, 4>(rounds, kind));
+}
+BeamKernelFn PickLong48(uint32_t rounds, int kind, bool late) { return PickLongOf<48>(rounds, kind, late); }
+}  // namespace tann

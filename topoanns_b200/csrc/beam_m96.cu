@@ -1,0 +1,10 @@
+// The beam-search kernels for 96 chunks.
+#include "beam_long.cuh"
+#include "beam_short.cuh"
+
+namespace tann {
+BeamKernelFn PickShort96(uint32_t rounds, int kind, uint32_t list_regs) {
+    return list_regs == 1 ? PickShortOf<96, 1>(rounds, kind) : (list_regs == 2 ? PickShortOf<96, 2>(rounds, kind) : PickShortOf<96, 4>(rounds, kind));
+}
+BeamKernelFn PickLong96(uint32_t rounds, int kind, bool late) { return PickLongOf<96>(rounds, kind, late); }
+}  // namespace tann

@@ -1,0 +1,112 @@
+// Which beam-search kernel serves a call, and with what shared memory.
+#include "beam_long.cuh"
+#include "beam_short.cuh"
+#include "tann_launch.h"
+
+namespace tann {
+
+BeamKernelFn PickShort32(uint32_t rounds, int kind, uint32_t list_regs);
+BeamKernelFn PickShort48(uint32_t rounds, int kind, uint32_t list_regs);
+BeamKernelFn PickShort96(uint32_t rounds, int kind, uint32_t list_regs);
+BeamKernelFn PickLong32(uint32_t rounds, int kind, bool late);
+BeamKernelFn PickLong48(uint32_t rounds, int kind, bool late);
+BeamKernelFn PickLong96(uint32_t rounds, int kind, bool late);
+
+// dims interleaved per pair of codes: [group of 32 (16) chunks][pair][chunk][dim of the chunk][code of the pair]
+__global__ void __launch_bounds__(256)
+pack_pivots_kernel(const float* __restrict__ col_major, uint32_t M, uint32_t sub, float* __restrict__ out) {
+    const uint64_t total = (uint64_t)M * sub * kCentroids;
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t chunk_group = (uint32_t)(e / ((uint64_t)32 * sub * kCentroids));
+        const uint32_t width = min(32u, M - chunk_group * 32);
+        uint64_t r = e - (uint64_t)chunk_group * 32 * sub * kCentroids;
+        const uint32_t code_bit = (uint32_t)(r & 1u); r >>= 1;
+        const uint32_t dim = (uint32_t)(r % sub); r /= sub;
+        const uint32_t m = (uint32_t)(r % width); r /= width;
+        const uint32_t code = 2u * (uint32_t)r + code_bit;
+        out[e] = __ldg(col_major + (size_t)((chunk_group * 32 + m) * sub + dim) * kCentroids + code);
+    }
+}
+
+bool CanPackPivots(uint32_t M, uint32_t dim) {
+    return (M == 32 || M == 48 || M == 96) && (dim == 2 * M || dim == 4 * M || dim == 8 * M);
+}
+
+cudaError_t LaunchPackPivots(const float* col_major, uint32_t M, uint32_t dim, float* out, cudaStream_t stream) {
+    pack_pivots_kernel<<<SmCount() * 2, 256, 0, stream>>>(col_major, M, dim / M, out);
+    return cudaGetLastError();
+}
+
+static uint32_t ResidentBlocks(uint32_t smem) { return (228u * 1024u) / (smem + 1024u + 512u); }
+
+bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan) {
+    const uint32_t M = ix.num_chunks, C = p.candidate_capacity, L = p.top_l;
+    const uint32_t slots = p.search_width * ix.degree;
+    const bool late = p.learned_stop.enabled != 0;
+    if (!(M == 32 || M == 48 || M == 96) || slots > 256u || L > 1024 || C > 1024 || ix.dim > kBloomWords) return false;
+    if (p.stop_prefix != 0 && p.stop_prefix < L) return false;
+    const bool sharded = ix.adjacency.num_shards > 1 || ix.codes.num_shards > 1;
+    const bool nbr = ix.neighbor_codes.base[0] != nullptr;
+    if ((sharded && (late || nbr)) || (nbr && ix.neighbor_codes.num_shards > 1)) return false;
+    plan->kind = sharded ? 2 : (nbr ? 1 : 0);
+    plan->rounds = slots > 128u ? 2u : 1u;
+    plan->late = late;
+    // the long form also repeats the queries the short form gives up on
+    plan->list_len = C;
+    const uint32_t one = LongLayout(M, plan->rounds, C, false).total, two = LongLayout(M, plan->rounds, C, true).total;
+    plan->two_lists = ResidentBlocks(two) == ResidentBlocks(one);
+    plan->long_smem = plan->two_lists ? two : one;
+    plan->smem = plan->long_smem;
+    if (plan->long_smem > 227u * 1024u - 512u) return false;
+    plan->list_regs = 0;
+    plan->pool_len = 0;
+    plan->may_mark = false;
+    if (L > 128 || late || ix.num_nodes > 0x3fffffffull) return true;
+    const uint32_t regs = L <= 32 ? 1u : (L <= 64 ? 2u : 4u);
+    if (C > 32 * regs) {
+        // room for the ranks behind the list, the keys of two pushes and some slack for the cut
+        const uint32_t want = C - 32 * regs + 64 + 256 * plan->rounds, most = kSlotThreads * kTailPer;
+        plan->pool_len = want < most ? want : most;
+        if (plan->pool_len < C - 32 * regs + 64 + 128 * plan->rounds) { plan->pool_len = 0; return true; }
+    }
+    const uint32_t smem = ShortLayout(M, plan->rounds, plan->pool_len).total;
+    if (smem > 227u * 1024u - 512u) { plan->pool_len = 0; return true; }
+    plan->list_regs = regs;
+    plan->may_mark = C > L;
+    plan->smem = smem;
+    return true;
+}
+
+static cudaError_t LaunchBeamKernel(BeamKernelFn k, const BeamArgs& a, uint32_t grid, uint32_t threads, uint32_t smem, cudaStream_t stream) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<grid, threads, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t LaunchFast(BeamArgs a, const FastPlan& plan, uint64_t num_queries, cudaStream_t stream) {
+    const uint32_t M = a.ix.num_chunks;
+    a.list_len = plan.list_len;
+    a.two_lists = plan.two_lists ? 1u : 0u;
+    a.pool_len = plan.pool_len;
+    a.only_marked = 0;
+    uint32_t long_grid = (uint32_t)num_queries;
+    if (plan.list_regs != 0) {
+        BeamKernelFn k = M == 32   ? PickShort32(plan.rounds, plan.kind, plan.list_regs)
+                         : M == 48 ? PickShort48(plan.rounds, plan.kind, plan.list_regs)
+                                   : PickShort96(plan.rounds, plan.kind, plan.list_regs);
+        const cudaError_t e = LaunchBeamKernel(k, a, (uint32_t)num_queries, kShortThreads, plan.smem, stream);
+        if (e != cudaSuccess || !plan.may_mark) return e;
+        a.only_marked = 1;
+        const uint32_t most = (uint32_t)SmCount();
+        long_grid = long_grid < most ? long_grid : most;
+    }
+    BeamKernelFn k = M == 32   ? PickLong32(plan.rounds, plan.kind, plan.late)
+                     : M == 48 ? PickLong48(plan.rounds, plan.kind, plan.late)
+                               : PickLong96(plan.rounds, plan.kind, plan.late);
+    return LaunchBeamKernel(k, a, long_grid, kBeamThreads, plan.long_smem, stream);
+}
+
+uint32_t FastBlocksPerSm(const FastPlan& plan) { return ResidentBlocks(plan.smem); }
+
+}  // namespace tann

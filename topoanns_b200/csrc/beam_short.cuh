@@ -1,0 +1,674 @@
+// Beam search for lists of at most 128 ranks in the traversal (top_l <= 128), chunk counts that are multiples of 16, at most
+// 256 frontier slots per step: the common case of the path. One query per block of five warps; the traversal is the
+// reference kernel's (src/search/topology_search_kernel.cu:2190-2664) step by step, and the records are bit for bit those of
+// the general kernels.
+//
+// A step ("push") is one dependent chain - memory round trip, visited filter, table sums, list, next memory round trip - and
+// with four or five queries per SM both the chain's length and the instructions it issues bound the kernel. Hence:
+//
+// * Four slot warps own the frontier slots (adjacency ids, code rows, visited filter, table sums). A fifth, the list warp,
+//   holds the sorted list in registers (kList keys per lane, rank = register * 32 + lane) and does the list work alone: no
+//   shared-memory list, no merge barriers, and each of its instructions is issued once instead of by every warp.
+// * Early selection. The next nodes are the smallest among the list's unexpanded entries (known before the push) and the
+//   push's new keys below the list's last one. The list warp picks them right behind the one barrier after the table sums;
+//   the slot warps issue the next loads and the list warp merges the new keys meanwhile: a sort of 32 keys across the
+//   lanes, one split against the end of the list and a bitonic merge.
+// * Lazy tail. Ranks from 32 * kList on never influence the traversal. When the caller wants a longer list they are kept in
+//   an unsorted pool, cut when it is full and sorted at the end.
+//
+// Keys: distance bits (order-preserving) << 32 | id << 2 | state, so that one 64-bit comparison orders copies of one node
+// (they have the same distance) as an eagerly merged list holds them: newest first. Copies within the first top_l ranks come
+// from one push only (anything else there is in the visited filter); when the last selected node has a twin that was not
+// selected, the twin becomes kTwin and stays behind it. Copies behind rank top_l are revisits: they are new (kNew) and lie in
+// front of the older, expanded ones. What the keys cannot tell is which copies an eagerly cut list drops when copies with
+// different states lie across its end; such a query (about one in 10^5) is marked in its statistics and searched again by
+// the general kernel.
+#pragma once
+
+#include "beam_table.cuh"
+
+namespace tann {
+
+constexpr uint32_t kSlotThreads = 128, kShortThreads = 160;
+constexpr uint32_t kNew = 0, kExpanded = 1, kTwin = 2;
+constexpr unsigned long long kNoKey = 0xff800000ffffffffull;   // (+inf, no id): behind every key
+constexpr uint32_t kTailBuckets = 128;
+constexpr int kTailPer = 6;            // the pool holds at most kSlotThreads * kTailPer keys
+
+__device__ __forceinline__ void SlotSync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void BlockSync() { asm volatile("bar.sync 0, 160;" ::: "memory"); }
+
+// Sorts one key per lane, descending.
+__device__ __forceinline__ unsigned long long WarpSortDescending(unsigned long long k, uint32_t lane) {
+#pragma unroll
+    for (uint32_t size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(kFull, k, stride);
+            const bool keep_max = ((lane & stride) == 0) == ((lane & size) == 0 || size == 32);
+            if ((o > k) == keep_max) k = o;
+        }
+    }
+    return k;
+}
+
+// Merges 32 keys (one per lane, descending) into the ascending list; returns the 32 largest of both (in no order).
+template <int kList>
+__device__ __forceinline__ unsigned long long MergeIntoList(unsigned long long (&list)[kList], unsigned long long k, uint32_t lane) {
+    // list's last 32 ascending against the new keys descending: the smaller halves, with the rest, form a bitonic sequence
+    const bool less = k < list[kList - 1];
+    const unsigned long long out = less ? list[kList - 1] : k;
+    if (less) list[kList - 1] = k;
+#pragma unroll
+    for (int stride = kList / 2; stride > 0; stride >>= 1) {
+#pragma unroll
+        for (int r = 0; r < kList; ++r) {
+            if ((r & stride) == 0) {
+                const unsigned long long x = list[r], y = list[r + stride];
+                const bool swap = y < x;
+                list[r] = swap ? y : x;
+                list[r + stride] = swap ? x : y;
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t stride = 16; stride > 0; stride >>= 1) {
+        const bool keep_max = (lane & stride) != 0;
+#pragma unroll
+        for (int r = 0; r < kList; ++r) {
+            const unsigned long long o = __shfl_xor_sync(kFull, list[r], stride);
+            if ((o > list[r]) == keep_max) list[r] = o;
+        }
+    }
+    return out;
+}
+
+__device__ __forceinline__ Cand RecordOf(unsigned long long k) {
+    Cand c;
+    c.dist = FromOrderedBits((uint32_t)(k >> 32));
+    const uint32_t low = (uint32_t)k;
+    c.id = low == 0xffffffffu ? kInvalid : (low >> 2) | ((low & 3u) == kExpanded ? kExpandedBit : 0u);
+    return c;
+}
+
+// ---- the tail --------------------------------------------------------------------------------------------------------------
+struct TailScratch {
+    uint32_t* hist;     // [kTailBuckets + 1]
+    uint32_t* range;    // [2]
+    uint32_t* counts;   // [32]
+};
+
+__device__ __forceinline__ uint32_t TailBucket(unsigned long long k, uint32_t lo, uint32_t inv) {
+    const uint32_t off = (uint32_t)(k >> 32) - lo;
+    return min(inv == 0u ? off : __umulhi(off, inv), kTailBuckets - 1u);
+}
+
+// Cuts the n keys of the pool to the smallest `room` (a few more where keys fall into one bucket: only whole buckets of the
+// distance are dropped, so every copy of a kept key is kept) and, at the end of the search (`sort`), sorts them.
+// Returns the number of keys kept; *bound gets the largest distance bits kept. The slot warps call.
+static __device__ __noinline__ uint32_t CutTail(unsigned long long* pool, const TailScratch s, uint32_t n, uint32_t room, bool sort,
+                                         uint32_t* bound) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    static_assert(kTailBuckets == kSlotThreads, "one bucket counter per thread");
+    uint32_t lo = 0xffffffffu, hi = 0;
+    if (tid < 2) s.range[tid] = tid == 0 ? 0xffffffffu : 0u;
+    SlotSync();
+#pragma unroll 1
+    for (uint32_t i = tid; i < n; i += kSlotThreads) {
+        const uint32_t b = (uint32_t)(pool[i] >> 32);
+        lo = min(lo, b);
+        hi = max(hi, b);
+    }
+    lo = __reduce_min_sync(kFull, lo);
+    hi = __reduce_max_sync(kFull, hi);
+    if (lane == 0) { atomicMin(&s.range[0], lo); atomicMax(&s.range[1], hi); }
+    SlotSync();
+    lo = s.range[0];
+    hi = s.range[1];
+    uint32_t inv = 0, kept = n;
+    // Distances are spread unevenly (the first entries lie far out), so the range is narrowed to the buckets that are kept
+    // until these hold little more than `room` keys.
+#pragma unroll 1
+    for (int pass = 0; pass < 4; ++pass) {
+        const uint32_t range = hi - lo;
+        // bucket = (bits - lo) * kTailBuckets / (range + 1), rounded down: monotone in the distance
+        inv = range < kTailBuckets ? 0u : (uint32_t)(((unsigned long long)kTailBuckets << 32) / ((unsigned long long)range + 1));
+        s.hist[tid] = 0;
+        SlotSync();
+#pragma unroll 1
+        for (uint32_t i = tid; i < n; i += kSlotThreads) {
+            const unsigned long long k = pool[i];
+            if ((uint32_t)(k >> 32) <= hi) atomicAdd(&s.hist[TailBucket(k, lo, inv)], 1u);
+        }
+        SlotSync();
+        // every warp: the first bucket with `room` keys up to its end (four buckets per lane)
+        const uint4 c = reinterpret_cast<const uint4*>(s.hist)[lane];
+        const uint32_t sum = c.x + c.y + c.z + c.w;
+        uint32_t incl = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, off);
+            if (lane >= (uint32_t)off) incl += t;
+        }
+        const uint32_t all = __shfl_sync(kFull, incl, 31);
+        uint32_t last = kTailBuckets - 1u, upto = all;
+        if (all > room) {
+            const uint32_t owner = __ffs(__ballot_sync(kFull, incl >= room)) - 1u;
+            uint32_t run = incl - sum, b = 0;
+            run += c.x;
+            if (run < room) { b = 1; run += c.y; }
+            if (run < room) { b = 2; run += c.z; }
+            if (run < room) { b = 3; run += c.w; }
+            last = __shfl_sync(kFull, lane * 4u + b, owner);
+            upto = __shfl_sync(kFull, run, owner);
+        }
+        kept = upto;
+        if (last == kTailBuckets - 1u) break;
+        // the largest offset of bucket `last`: off * inv < (last + 1) << 32
+        hi = lo + (inv == 0u ? last : (uint32_t)((((unsigned long long)(last + 1u) << 32) - 1u) / inv));
+        if (inv == 0u || kept <= room + 32u) break;
+        SlotSync();   // the counters are read before they are cleared
+    }
+    *bound = hi;
+    SlotSync();
+    // the keys that stay, in the pool's order
+    unsigned long long k[kTailPer];
+    uint32_t stays = 0;
+#pragma unroll
+    for (int u = 0; u < kTailPer; ++u) {
+        const uint32_t i = tid + u * kSlotThreads;
+        bool stay = false;
+        if (u * kSlotThreads < n) {
+            if (i < n) { k[u] = pool[i]; stay = (uint32_t)(k[u] >> 32) <= hi; }
+            const uint32_t b = __ballot_sync(kFull, stay);
+            if (lane == 0) s.counts[u * 4 + warp] = __popc(b);
+        } else if (lane == 0) {
+            s.counts[u * 4 + warp] = 0;
+        }
+        stays |= (stay ? 1u : 0u) << u;
+    }
+    SlotSync();
+    const uint32_t mine = lane < 4u * kTailPer ? s.counts[lane] : 0u;
+#pragma unroll
+    for (int u = 0; u < kTailPer; ++u) {
+        if (u * kSlotThreads < n) {
+            const bool stay = (stays >> u) & 1u;
+            const uint32_t b = __ballot_sync(kFull, stay);
+            const uint32_t before = __reduce_add_sync(kFull, lane < u * 4u + warp ? mine : 0u);
+            if (stay) pool[before + __popc(b & ((1u << lane) - 1u))] = k[u];
+        }
+    }
+    kept = __reduce_add_sync(kFull, mine);
+    s.hist[tid] = 0;
+    SlotSync();
+    if (!sort) return kept;
+    // ---- bucket sort of the kept keys ------------------------------------------------------------------------------------
+    {
+        const uint32_t range = hi - lo;
+        inv = range < kTailBuckets ? 0u : (uint32_t)(((unsigned long long)kTailBuckets << 32) / ((unsigned long long)range + 1));
+    }
+    uint32_t slot[kTailPer];
+#pragma unroll
+    for (int u = 0; u < kTailPer; ++u) {
+        const uint32_t i = tid + u * kSlotThreads;
+        if (i < kept) {
+            k[u] = pool[i];
+            slot[u] = atomicAdd(&s.hist[TailBucket(k[u], lo, inv)], 1u);
+        }
+    }
+    SlotSync();
+    if (warp == 0) {
+        const uint4 c = reinterpret_cast<const uint4*>(s.hist)[lane];
+        const uint32_t sum = c.x + c.y + c.z + c.w;
+        uint32_t incl = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, off);
+            if (lane >= (uint32_t)off) incl += t;
+        }
+        const uint32_t run = incl - sum;
+        reinterpret_cast<uint4*>(s.hist)[lane] = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
+        if (lane == 31) s.hist[kTailBuckets] = incl;
+    }
+    SlotSync();
+#pragma unroll
+    for (int u = 0; u < kTailPer; ++u) {
+        const uint32_t i = tid + u * kSlotThreads;
+        if (i < kept) {
+            const uint32_t p = s.hist[TailBucket(k[u], lo, inv)] + slot[u];
+            pool[p] = k[u];
+        }
+    }
+    SlotSync();
+#pragma unroll
+    for (int u = 0; u < kTailPer; ++u) {
+        const uint32_t i = tid + u * kSlotThreads;
+        if (i < kept) {
+            const uint32_t bk = TailBucket(k[u], lo, inv);
+            const uint32_t b = s.hist[bk], e = s.hist[bk + 1];
+            const uint32_t own = b + slot[u];   // equal keys in the order they were scattered in
+            uint32_t r = b;
+#pragma unroll 1
+            for (uint32_t j = b; j < e; ++j) r += (pool[j] < k[u] || (pool[j] == k[u] && j < own)) ? 1u : 0u;
+            slot[u] = r;
+        }
+    }
+    SlotSync();
+#pragma unroll
+    for (int u = 0; u < kTailPer; ++u)
+        if (tid + u * kSlotThreads < kept) pool[slot[u]] = k[u];
+    SlotSync();
+    return kept;
+}
+
+
+struct ShortLayout {
+    uint32_t bloom, fkey, pool, total;
+    __host__ __device__ ShortLayout(uint32_t M, uint32_t rounds, uint32_t pool_len) {
+        bloom = M * kCentroids * 4;
+        fkey = bloom + kBloomWords * 4;                      // new keys of a push, two pushes in turn
+        pool = fkey + 2 * kSlotThreads * rounds * 8;
+        total = pool + pool_len * 8;
+    }
+};
+
+// kKind: 0 = codes gathered by id, 1 = neighbour-code layout, 2 = codes and adjacency in node-id-range shards.
+// kR: slots per thread (ceil(W * degree / 128)). kList: list registers per lane of the list warp.
+template <int kM, int kR, int kKind, int kList>
+__global__ void __launch_bounds__(kShortThreads, kM <= 32 ? 5 : (kM <= 48 ? 4 : (kM <= 64 ? 3 : 2)))
+beam_short_kernel(const __grid_constant__ BeamArgs a) {
+    constexpr bool kNbr = kKind == 1;
+    constexpr bool kOneShard = kKind != 2;
+    constexpr uint32_t kFresh = kSlotThreads * kR;   // new keys per push at most
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const ShortLayout lay(kM, kR, a.pool_len);
+    uint32_t* bloom = reinterpret_cast<uint32_t*>(smem_raw + lay.bloom);
+    unsigned long long* fkey = reinterpret_cast<unsigned long long*>(smem_raw + lay.fkey);
+    unsigned long long* pool = reinterpret_cast<unsigned long long*>(smem_raw + lay.pool);
+    __shared__ unsigned long long s_thr;       // last key of the list; a new key behind it cannot enter
+    __shared__ uint32_t s_count;               // new keys of the push | passing slots << 16
+    __shared__ uint32_t s_pool_n, s_tail_thr, s_fail, s_range[2];
+    __shared__ uint32_t s_nsel, s_cut;         // nodes selected (0 ends the search); the pool is to be cut
+    __shared__ uint32_t s_node[TANN_MAX_SEARCH_WIDTH];
+    const uint64_t q = blockIdx.x;
+    const uint32_t W = a.p.search_width, deg = a.ix.degree, slots = W * deg;
+    const uint32_t entry_begin = a.entry_offsets[q];
+    const uint32_t num_entries = a.entry_offsets[q + 1] - entry_begin;
+    const uint32_t entry_pushes = (num_entries + slots - 1) / slots;
+    const bool tail = a.pool_len != 0;
+    const uint32_t C = a.p.candidate_capacity;
+
+    if (warp < 4) {
+        // ================================================ slot warps ========================================================
+        const uint64_t N = a.ix.num_nodes;
+        const uint32_t lt = (1u << lane) - 1u;
+        uint32_t my_k[kR], my_j[kR];          // this thread's slots: node my_k, neighbour my_j
+        uint32_t id[kR], words[kR][kM / 4];
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            const uint32_t s = r * kSlotThreads + tid;
+            my_k[r] = s / deg;
+            my_j[r] = s - my_k[r] * deg;
+            id[r] = (s < slots && s < num_entries) ? __ldg(a.entry_ids + entry_begin + s) : kInvalid;
+        }
+        {
+            const uint32_t d = a.ix.dim;
+            float* lut = reinterpret_cast<float*>(smem_raw);
+            float* sq = reinterpret_cast<float*>(bloom);   // dim <= kBloomWords (checked by the launcher)
+            const float* given = a.lut != nullptr ? a.lut + q * (uint64_t)kM * kCentroids : nullptr;
+            if (given == nullptr)   // src/search/pq_query_tables.cu:33-52
+                for (uint32_t i = tid; i < d; i += kSlotThreads)
+                    sq[i] = LoadAsFloat<float>(a.queries, a.query_kind, q * d + i) - __ldg(a.ix.pq_centroid + i);
+            SlotSync();
+            if (given == nullptr && a.pivots_packed != nullptr && d == 2 * kM) TableFromPacked<kM, 2>(lut, sq, a.pivots_packed, tid);
+            else if (given == nullptr && a.pivots_packed != nullptr && d == 4 * kM) TableFromPacked<kM, 4>(lut, sq, a.pivots_packed, tid);
+            else if (given == nullptr && a.pivots_packed != nullptr && d == 8 * kM) TableFromPacked<kM, 8>(lut, sq, a.pivots_packed, tid);
+            else TableFromColumns<kM>(lut, sq, a, given, tid);
+            SlotSync();
+        }
+        for (uint32_t i = tid; i < kBloomWords / 4; i += kSlotThreads) reinterpret_cast<uint4*>(bloom)[i] = make_uint4(0, 0, 0, 0);
+        const LaneOffsets offs(lane);
+        BlockSync();
+        uint32_t push = 0, hash_iter = 0, nslots = slots;
+        while (entry_pushes != 0) {
+            // ---- visited tests, table sums -----------------------------------------------------------------------------------
+            if (!kNbr || push < entry_pushes) {
+#pragma unroll
+                for (int r = 0; r < kR; ++r)
+                    if (id[r] < N) LoadCodesXor<kM>(Row<kOneShard>(a.ix.codes, id[r], kM), lane, words[r]);
+            }
+            BloomBits bits[kR];
+            bool pass[kR];
+            unsigned long long key[kR];
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                bits[r] = BloomPositions(id[r]);
+                pass[r] = id[r] < N;
+                // an id that is neither the padding value nor a node of the index is skipped and reported
+                if (id[r] != kInvalid && !pass[r] && a.status != nullptr) atomicOr(a.status, TANN_STATUS_BEAM_ID_RANGE);
+            }
+            if (hash_iter == 0 && push != 0) BlockSync();   // the list warp has rebuilt the filter
+            pass[0] = pass[0] && !BloomTest(bits[0], bloom);
+            bool first_added = false;
+            if constexpr (kR > 1) {
+                if (nslots > kSlotThreads) {
+                    // the reference's 128 threads walk the slots in rounds of 128: the tests of a round see the adds of the
+                    // rounds before it (src/search/topology_search_kernel.cu:2543-2564)
+                    SlotSync();
+                    if (pass[0]) BloomAdd(bits[0], bloom);
+                    SlotSync();
+                    first_added = true;
+                    pass[1] = pass[1] && !BloomTest(bits[1], bloom);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                PermuteXor<kM>(lane, words[r]);
+                key[r] = ((unsigned long long)OrderedBits(AdcXor<kM>(smem_raw, words[r], offs)) << 32) | (id[r] << 2);
+            }
+            // ---- which new keys go to the list, which into the tail ----------------------------------------------------------
+            // (a threshold from before the last merge is an upper bound: the list warp sorts out the rest)
+            const unsigned long long thr = *reinterpret_cast<volatile unsigned long long*>(&s_thr);
+            uint32_t to_list[kR], to_tail[kR], mine = 0, mine_tail = 0;
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                const bool surv = pass[r] && key[r] < thr;
+                to_list[r] = __ballot_sync(kFull, surv);
+                mine += __popc(to_list[r]) + (__popc(__ballot_sync(kFull, pass[r])) << 16);
+                to_tail[r] = 0;
+                if (tail) {
+                    to_tail[r] = __ballot_sync(kFull, pass[r] && !surv && (uint32_t)(key[r] >> 32) <= s_tail_thr);
+                    mine_tail += __popc(to_tail[r]);
+                }
+            }
+            uint32_t base = 0, base_tail = 0;
+            if (lane == 0) {
+                if (mine != 0) base = atomicAdd(&s_count, mine);
+                if (tail && mine_tail != 0) base_tail = atomicAdd(&s_pool_n, mine_tail);
+            }
+            base = __shfl_sync(kFull, base, 0) & 0xffffu;
+            unsigned long long* fresh = fkey + (push & 1u) * kFresh;
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                if ((to_list[r] >> lane) & 1u) fresh[base + (r == 1 ? __popc(to_list[0]) : 0u) + __popc(to_list[r] & lt)] = key[r];
+            }
+            if (tail) {
+                base_tail = __shfl_sync(kFull, base_tail, 0);
+#pragma unroll
+                for (int r = 0; r < kR; ++r) {
+                    if ((to_tail[r] >> lane) & 1u) {
+                        const uint32_t at = base_tail + (r == 1 ? __popc(to_tail[0]) : 0u) + __popc(to_tail[r] & lt);
+                        if (at < a.pool_len) pool[at] = key[r];   // (an overflow is seen by the list warp)
+                    }
+                }
+            }
+            BlockSync();
+            // ---- visited marks, while the list warp selects -------------------------------------------------------------------
+            ++push;
+            if (++hash_iter >= 3) {
+                // every third merge the filter is rebuilt from the first top_l ranks (:2394-2411,2636-2654); this push's marks
+                // would be wiped with the rest
+                hash_iter = 0;
+#pragma unroll 2
+                for (uint32_t i = tid; i < kBloomWords / 4; i += kSlotThreads) reinterpret_cast<uint4*>(bloom)[i] = make_uint4(0, 0, 0, 0);
+            } else {
+#pragma unroll
+                for (int r = 0; r < kR; ++r)
+                    if (pass[r] && !(kR > 1 && r == 0 && first_added)) BloomAdd(bits[r], bloom);
+            }
+            BlockSync();
+            // ---- the next push's loads ---------------------------------------------------------------------------------------
+            if (push < entry_pushes) {
+#pragma unroll
+                for (int r = 0; r < kR; ++r) {
+                    const uint32_t s = r * kSlotThreads + tid, e = push * slots + s;
+                    id[r] = (s < slots && e < num_entries) ? __ldg(a.entry_ids + entry_begin + e) : kInvalid;
+                }
+            } else {
+                const uint32_t nsel = s_nsel;
+                if (nsel == 0) break;
+                nslots = nsel * deg;
+#pragma unroll
+                for (int r = 0; r < kR; ++r) {
+                    id[r] = kInvalid;
+                    if (my_k[r] < nsel) {
+                        const uint32_t node = s_node[my_k[r]];
+                        const uint32_t* row = node < a.ix.adjacency_cached_rows
+                                                  ? a.ix.adjacency_cache + (uint64_t)node * deg
+                                                  : reinterpret_cast<const uint32_t*>(Row<kOneShard>(a.ix.adjacency, node, (uint64_t)deg * 4));
+                        id[r] = __ldg(row + my_j[r]);
+                        // the slot's code row sits at (node, j): both loads share one round trip
+                        if constexpr (kNbr)
+                            LoadCodesXor<kM>(Row<kOneShard>(a.ix.neighbor_codes, node, (uint64_t)deg * kM) + (size_t)my_j[r] * kM, lane, words[r]);
+                    }
+                }
+            }
+            if (tail && s_cut != 0u) {
+                // scratch: the next push's place for new keys
+                uint32_t* free_words = reinterpret_cast<uint32_t*>(fkey + (push & 1u) * kFresh);
+                uint32_t bound;
+                const uint32_t kept = CutTail(pool, TailScratch{free_words, s_range, free_words + kTailBuckets + 4}, min(s_pool_n, a.pool_len), C - 32u * kList, false, &bound);
+                if (tid == 0) { s_pool_n = kept; s_tail_thr = bound; }
+                BlockSync();
+            }
+        }
+        // ---- results: the ranks behind the list --------------------------------------------------------------------------------
+        if (entry_pushes == 0) {
+            for (uint32_t i = tid; i < C; i += kSlotThreads) a.out_cand[q * (uint64_t)C + i] = RecordOf(kNoKey);
+            if (tid < 8) a.out_stats[q * 8 + tid] = tid == 5 ? 0xffffffffu : 0u;
+            return;
+        }
+        if (tail) {
+            BlockSync();   // the list warp's last merge
+            const uint32_t room = C - 32u * kList;
+            uint32_t n = min(s_pool_n, a.pool_len), fail = s_fail;
+            if (n != 0) {
+                uint32_t bound;
+                uint32_t* words32 = reinterpret_cast<uint32_t*>(fkey);
+                n = CutTail(pool, TailScratch{words32, s_range, words32 + kTailBuckets + 4}, n, room, true, &bound);
+                // copies of one node across the end of the list, in different states
+                if (n > room && (pool[room - 1] >> 2) == (pool[room] >> 2)) {
+                    uint32_t b = room, e = room;
+                    while (b > 0 && (pool[b - 1] >> 2) == (pool[room] >> 2)) --b;
+                    while (e < n && (pool[e] >> 2) == (pool[room] >> 2)) ++e;
+                    if (pool[b] != pool[e - 1]) fail = 1;   // ascending: the states differ exactly when first and last do
+                }
+            }
+            Cand* out = a.out_cand + q * (uint64_t)C + 32u * kList;
+            for (uint32_t i = tid; i < room; i += kSlotThreads) out[i] = RecordOf(i < n ? pool[i] : kNoKey);
+            if (tid == 0 && fail != 0u) a.out_stats[q * 8 + 6] = 1u;
+        }
+    } else {
+        // ================================================ list warp =========================================================
+        const uint32_t L = a.p.top_l, cap = min(C, 32u * kList);   // ranks kept here
+        unsigned long long list[kList];
+#pragma unroll
+        for (int r = 0; r < kList; ++r) list[r] = kNoKey;
+        if (lane == 0) {
+            s_thr = kNoKey;
+            s_count = 0; s_pool_n = 0; s_tail_thr = 0xffffffffu; s_fail = 0; s_nsel = 0; s_cut = 0;
+        }
+        uint32_t valid = 0, visited = 0, expanded = 0, iterations = 0, first_full = 0xffffffffu, hash_iter = 0, fail = 0;
+        // lane x: the x-th unexpanded entry of the list, and its rank
+        unsigned long long un_key = kNoKey;
+        uint32_t un_pos = 0;
+        BlockSync();
+        for (uint32_t push = 0; entry_pushes != 0; ++push) {
+            BlockSync();   // the push's new keys are there
+            unsigned long long* fresh = fkey + (push & 1u) * kFresh;
+            const uint32_t counts = s_count, n = counts & 0xffffu, fv = counts >> 16;
+            const uint32_t pool_n = tail ? s_pool_n : 0u;
+            const uint32_t nv = (uint32_t)min((uint64_t)C, (uint64_t)valid + fv);
+            if (first_full == 0xffffffffu && nv >= L) first_full = push < entry_pushes ? 0u : iterations;
+            visited += fv;
+            valid = nv;
+            const bool more = push + 1 < entry_pushes;   // the next push takes entries again
+            // ---- selection -----------------------------------------------------------------------------------------------------
+            unsigned long long k0 = lane < n ? fresh[lane] : kNoKey;   // new keys [0, 32)
+            uint32_t nsel = 0, list_end = 0;
+            unsigned long long last_pick = 0;
+            if (!more && expanded < a.p.max_expansions) {
+                unsigned long long least = k0;
+                uint32_t at = lane, pick = 0, un_taken = 0, new_picks = 0;
+#pragma unroll 1
+                for (uint32_t i = 32u + lane; i < n; i += 32u) {
+                    const unsigned long long k = fresh[i];
+                    if (k < least) { least = k; at = i; }
+                }
+                unsigned long long s_min = n != 0 ? WarpMinKey(least) : kNoKey;
+#pragma unroll 1
+                while (nsel < W) {
+                    const unsigned long long u = __shfl_sync(kFull, un_key, un_taken);
+                    if (s_min < u) {
+                        // inside the first L ranks?
+                        uint32_t below = new_picks;
+#pragma unroll
+                        for (int r = 0; r < kList; ++r) below += __popc(__ballot_sync(kFull, list[r] < s_min));
+                        if (below >= L) break;
+                        if (lane == nsel) pick = (uint32_t)s_min >> 2;
+                        last_pick = s_min;
+                        ++nsel;
+                        ++new_picks;
+                        const uint32_t owner = __ffs(__ballot_sync(kFull, least == s_min)) - 1u;
+                        if (lane == owner) {   // selected: expanded from now on
+                            if (at < 32u) k0 |= kExpanded; else fresh[at] = least | kExpanded;
+                            least = kNoKey;
+                            if (n > 32u) {
+                                if (lane < n && (k0 & 3u) == kNew) { least = k0; at = lane; }
+#pragma unroll 1
+                                for (uint32_t i = 32u + lane; i < n; i += 32u) {
+                                    const unsigned long long k = fresh[i];
+                                    if ((k & 3u) == kNew && k < least) { least = k; at = i; }
+                                }
+                            }
+                        }
+                        if (nsel < W) s_min = WarpMinKey(least);
+                    } else if (u < kNoKey) {
+                        const uint32_t pos = __shfl_sync(kFull, un_pos, un_taken);
+                        if (pos + new_picks >= L) break;
+                        if (lane == nsel) pick = (uint32_t)u >> 2;
+                        last_pick = u;
+                        list_end = pos + 1u;
+                        ++un_taken;
+                        ++nsel;
+                    } else {
+                        break;
+                    }
+                }
+                if (lane < nsel) s_node[lane] = pick;
+                if (nsel != 0) ++iterations;
+                expanded += nsel;
+            }
+            // the pool must take this push's displaced entries and the next push's tail keys
+            const bool cut = tail && pool_n + n + kFresh > a.pool_len;
+            if (lane == 0) {
+                s_nsel = nsel;
+                s_count = 0;
+                s_cut = cut ? 1u : 0u;
+            }
+            if (tail && pool_n > a.pool_len) fail = 1;
+            BlockSync();   // the selection is there
+            const bool last_push = !more && nsel == 0;
+            if (cut && !last_push) BlockSync();
+            // ---- merge, behind the next push's loads ------------------------------------------------------------------------------
+            if (list_end != 0u) {   // every unexpanded entry up to there was selected
+#pragma unroll
+                for (int r = 0; r < kList; ++r)
+                    if (r * 32u + lane < list_end) list[r] = (list[r] & ~3ull) | kExpanded;
+            }
+            if (nsel != 0u) {   // a twin of the last selected node that was not selected stays behind it
+#pragma unroll
+                for (int r = 0; r < kList; ++r)
+                    if ((list[r] >> 2) == (last_pick >> 2) && (list[r] & 3u) == kNew) list[r] |= kTwin;
+                if ((k0 >> 2) == (last_pick >> 2) && (k0 & 3u) == kNew) k0 |= kTwin;
+#pragma unroll 1
+                for (uint32_t i = 32u + lane; i < n; i += 32u)
+                    if ((fresh[i] >> 2) == (last_pick >> 2) && (fresh[i] & 3u) == kNew) fresh[i] |= kTwin;
+            }
+#pragma unroll 1
+            for (uint32_t c = 0; c < n; c += 32u) {
+                if (c != 0) k0 = c + lane < n ? fresh[c + lane] : kNoKey;
+                unsigned long long out = MergeIntoList<kList>(list, WarpSortDescending(k0, lane), lane);
+                if (tail) {
+                    const uint32_t b = __ballot_sync(kFull, out != kNoKey);
+                    if (b != 0u) {
+                        uint32_t at = 0;
+                        if (lane == 0) at = atomicAdd(&s_pool_n, (uint32_t)__popc(b));
+                        at = __shfl_sync(kFull, at, 0);
+                        if (at + (uint32_t)__popc(b) > a.pool_len) fail = 1;
+                        at += __popc(b & ((1u << lane) - 1u));
+                        if (out != kNoKey && at < a.pool_len) pool[at] = out;
+                    }
+                } else {
+                    if (cap < 32u * kList) {   // a list shorter than the registers hold
+                        const unsigned long long last = __shfl_sync(kFull, list[0], cap - 1u);
+                        if (C > L && __any_sync(kFull, out != kNoKey && (out >> 2) == (last >> 2) && out != last)) fail = 1;
+                        if (lane >= cap) { out = list[0]; list[0] = kNoKey; }
+                    }
+                    if (C > L) {
+                        // copies of one node across the end of the list, in different states
+                        const uint32_t end = cap - 1u;
+                        const unsigned long long last = __shfl_sync(kFull, list[kList - 1], end & 31u);
+                        if (__any_sync(kFull, out != kNoKey && (out >> 2) == (last >> 2) && out != last)) fail = 1;
+                    }
+                }
+            }
+            if (last_push) break;
+            if (n != 0) {
+                const unsigned long long last = __shfl_sync(kFull, list[kList - 1], (cap - 1u) & 31u);
+                if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(&s_thr) = last;
+            }
+            if (++hash_iter >= 3) {
+                hash_iter = 0;
+#pragma unroll
+                for (int r = 0; r < kList; ++r)
+                    if (r * 32u + lane < L && list[r] != kNoKey) BloomAdd((uint32_t)list[r] >> 2, bloom);
+                BlockSync();   // the filter is complete
+            }
+            // the first W unexpanded ranks below L
+            {
+                uint32_t found = 0;
+                un_key = kNoKey;
+#pragma unroll
+                for (int r = 0; r < kList; ++r) {
+                    uint32_t b = __ballot_sync(kFull, r * 32u + lane < L && list[r] != kNoKey && (list[r] & 3u) != kExpanded);
+#pragma unroll 1
+                    while (b != 0u && found < W) {
+                        const uint32_t src = __ffs(b) - 1u;
+                        const unsigned long long k = __shfl_sync(kFull, list[r], src);
+                        if (lane == found) { un_key = k; un_pos = r * 32u + src; }
+                        b &= b - 1u;
+                        ++found;
+                    }
+                }
+            }
+        }
+        if (entry_pushes == 0) return;
+        // ---- results: the list's ranks -----------------------------------------------------------------------------------------
+        Cand* out = a.out_cand + q * (uint64_t)C;
+#pragma unroll
+        for (int r = 0; r < kList; ++r)
+            if (r * 32u + lane < cap) out[r * 32u + lane] = RecordOf(list[r]);
+        if (lane == 0) {
+            uint32_t* st = a.out_stats + q * 8;
+            st[0] = visited; st[1] = expanded; st[2] = 0; st[3] = iterations;
+            st[4] = valid; st[5] = first_full; st[7] = 0;
+            st[6] = fail;   // the slot warps may set it once more, behind the next barrier
+            s_fail = fail;
+            __threadfence_block();
+        }
+        if (tail) BlockSync();
+        for (uint32_t i = 32u * kList + lane; !tail && i < C; i += 32u) out[i] = RecordOf(kNoKey);
+    }
+}
+
+typedef void (*BeamKernelFn)(const BeamArgs);
+template <int kM, int kList>
+BeamKernelFn PickShortOf(uint32_t rounds, int kind) {
+    if (rounds == 1)
+        return kind == 2 ? beam_short_kernel<kM, 1, 2, kList> : (kind == 1 ? beam_short_kernel<kM, 1, 1, kList> : beam_short_kernel<kM, 1, 0, kList>);
+    return kind == 2 ? beam_short_kernel<kM, 2, 2, kList> : (kind == 1 ? beam_short_kernel<kM, 2, 1, kList> : beam_short_kernel<kM, 2, 0, kList>);
+}
+
+}  // namespace tann

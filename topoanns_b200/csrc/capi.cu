@@ -103,16 +103,24 @@ TannStatus CheckBeam(const TannIndexView* ix, const TannBeamParams* p) {
 }
 
 struct BeamPlan {
+    bool fast_form;
+    tann::FastPlan fast;
     uint32_t F;
     size_t smem;
     int blocks_per_sm;
     uint32_t grid;
 };
 
-TannStatus PlanBeam(const TannIndexView* ix, const TannBeamParams* p, bool lut_in_kernel, uint64_t Q,
-                    BeamPlan* plan) {
-    (void)lut_in_kernel;
+TannStatus PlanBeam(const TannIndexView* ix, const TannBeamParams* p, uint64_t Q, BeamPlan* plan) {
     const uint32_t slots = p->search_width * ix->degree;
+    plan->fast_form = tann::PlanFast(*ix, *p, &plan->fast) && Q <= 0x7fffffffull;
+    if (Q == ~0ull) plan->fast_form = tann::PlanFast(*ix, *p, &plan->fast);
+    if (plan->fast_form) {
+        plan->smem = plan->fast.smem;
+        plan->blocks_per_sm = (int)tann::FastBlocksPerSm(plan->fast);
+        plan->grid = Q == ~0ull ? (uint32_t)(tann::SmCount() * plan->blocks_per_sm) : (uint32_t)Q;
+        return TANN_OK;
+    }
     plan->F = NextPow2(slots == 0 ? 1 : slots);
     plan->smem = tann::BeamSmemBytes(ix->num_chunks, p->candidate_capacity, plan->F, p->top_l, ix->dim);
     int dev = 0, max_optin = 0;
@@ -173,8 +181,10 @@ TannStatus tann_lut_build(const float* tables_col_major, const float* centroid,
     return TANN_OK;
 }
 
-TannStatus tann_beam_search(const TannIndexView* index, const TannBeamParams* params, const float* lut,
-                            const void* queries, uint32_t query_kind, uint64_t num_queries,
+// pivots_packed: the index's pivots as LaunchPackPivots lays them out, or nullptr.
+static TannStatus BeamSearch(const TannIndexView* index, const TannBeamParams* params, const float* lut,
+                             const float* pivots_packed,
+                             const void* queries, uint32_t query_kind, uint64_t num_queries,
                             const uint32_t* entry_offsets, const uint32_t* entry_ids,
                             void* out_candidates, uint32_t* out_stats, uint32_t* status,
                             tann_stream_t stream) {
@@ -204,7 +214,7 @@ TannStatus tann_beam_search(const TannIndexView* index, const TannBeamParams* pa
         }
     }
     BeamPlan plan;
-    st = PlanBeam(index, params, lut == nullptr, num_queries, &plan);
+    st = PlanBeam(index, params, num_queries, &plan);
     if (st != TANN_OK) return st;
     tann::BeamArgs a;
     memset(&a, 0, sizeof(a));
@@ -220,8 +230,22 @@ TannStatus tann_beam_search(const TannIndexView* index, const TannBeamParams* pa
     a.out_cand = static_cast<tann::Cand*>(out_candidates);
     a.out_stats = out_stats;
     a.status = status;
+    a.pivots_packed = pivots_packed;
+    if (plan.fast_form) {
+        TANN_CUDA(tann::LaunchFast(a, plan.fast, num_queries, (cudaStream_t)stream));
+        return TANN_OK;
+    }
     TANN_CUDA(tann::LaunchBeam(a, plan.smem, plan.grid, (cudaStream_t)stream));
     return TANN_OK;
+}
+
+TannStatus tann_beam_search(const TannIndexView* index, const TannBeamParams* params, const float* lut,
+                            const void* queries, uint32_t query_kind, uint64_t num_queries,
+                            const uint32_t* entry_offsets, const uint32_t* entry_ids,
+                            void* out_candidates, uint32_t* out_stats, uint32_t* status,
+                            tann_stream_t stream) {
+    return BeamSearch(index, params, lut, nullptr, queries, query_kind, num_queries, entry_offsets, entry_ids,
+                      out_candidates, out_stats, status, stream);
 }
 
 TannStatus tann_beam_search_occupancy(const TannIndexView* index, const TannBeamParams* params,
@@ -230,7 +254,8 @@ TannStatus tann_beam_search_occupancy(const TannIndexView* index, const TannBeam
     TannStatus st = CheckBeam(index, params);
     if (st != TANN_OK) return st;
     BeamPlan plan;
-    st = PlanBeam(index, params, lut_in_kernel != 0, ~0ull, &plan);
+    (void)lut_in_kernel;
+    st = PlanBeam(index, params, ~0ull, &plan);
     if (st != TANN_OK) return st;
     if (smem_bytes) *smem_bytes = (uint32_t)plan.smem;
     if (blocks_per_sm) *blocks_per_sm = (uint32_t)plan.blocks_per_sm;
@@ -674,6 +699,7 @@ struct TannSearcher {
     unsigned long long* d_counts;
     uint32_t* d_fixed_entries;   // max_entries ids: the fixed entry list before it is expanded per query
     uint32_t* d_status;          // TANN_STATUS_* bits of the last run
+    float* d_pivots;             // the PQ pivots laid out for the in-kernel table build (nullptr: other chunk shapes)
     uint32_t* h_status;
     // pinned staging
     // a batch that tann_searcher_submit enqueued and tann_searcher_wait has not collected yet
@@ -698,6 +724,7 @@ static void FreeSearcher(TannSearcher* s) {
     cudaFree(s->d_entry_ids); cudaFree(s->d_cand); cudaFree(s->d_cand_refined); cudaFree(s->d_stats);
     cudaFree(s->d_lut2); cudaFree(s->d_dists); cudaFree(s->d_ids); cudaFree(s->d_topk_dists);
     cudaFree(s->d_topk_ids); cudaFree(s->d_counts); cudaFree(s->d_fixed_entries); cudaFree(s->d_status);
+    cudaFree(s->d_pivots);
     cudaFreeHost(s->h_status);
     cudaFreeHost(s->h_queries); cudaFreeHost(s->h_topk_ids); cudaFreeHost(s->h_topk_dists);
     cudaFreeHost(s->h_stats); cudaFreeHost(s->h_entries);
@@ -742,6 +769,19 @@ TannStatus tann_searcher_create(const TannIndexView* index, uint64_t max_queries
     dev((void**)&s->d_counts, 16);
     dev((void**)&s->d_fixed_entries, (size_t)max_entries_per_query * 4);
     dev((void**)&s->d_status, 16);
+    bool equal_chunks = false;   // the packed layout is for chunks of one width
+    if (e == cudaSuccess && index->pq_tables_col_major != nullptr && index->pq_chunk_offsets != nullptr &&
+        tann::CanPackPivots(index->num_chunks, index->dim)) {
+        std::vector<uint32_t> offs(index->num_chunks + 1);
+        e = cudaMemcpy(offs.data(), index->pq_chunk_offsets, offs.size() * 4, cudaMemcpyDefault);
+        equal_chunks = e == cudaSuccess;
+        for (size_t m = 0; m < offs.size(); ++m) equal_chunks = equal_chunks && offs[m] == m * (index->dim / index->num_chunks);
+    }
+    if (equal_chunks) {
+        dev((void**)&s->d_pivots, d * 1024);
+        if (e == cudaSuccess) e = tann::LaunchPackPivots(index->pq_tables_col_major, index->num_chunks, index->dim, s->d_pivots, nullptr);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    }
     host((void**)&s->h_status, 16);
     host(&s->h_queries, Q * d * 4);
     host((void**)&s->h_topk_ids, Q * max_top_n * 4);
@@ -836,8 +876,8 @@ TannStatus tann_searcher_run_device(TannSearcher* s, const TannBeamParams* beam,
         ei = s->d_entry_ids;
     }
     // traversal, table built in the kernel
-    TannStatus st = tann_beam_search(&s->ix, beam, nullptr, queries_dev, query_kind, Q, eo, ei, s->d_cand,
-                                     s->d_stats, s->d_status, stream);
+    TannStatus st = BeamSearch(&s->ix, beam, nullptr, s->d_pivots, queries_dev, query_kind, Q, eo, ei, s->d_cand,
+                               s->d_stats, s->d_status, stream);
     if (st != TANN_OK) return st;
     const void* cand = s->d_cand;
     uint32_t capacity = beam->candidate_capacity;

@@ -16,6 +16,24 @@ size_t BeamSmemBytes(uint32_t M, uint32_t C, uint32_t F, uint32_t L, uint32_t d)
 cudaError_t LaunchBeam(const BeamArgs& a, size_t smem, uint32_t grid, cudaStream_t stream);
 cudaError_t BeamOccupancy(uint32_t M, uint32_t slots, size_t smem, int* blocks_per_sm);
 
+// The kernels for chunk counts of 32, 48 and 96 and up to 256 slots per step (beam_short.cuh, beam_long.cuh).
+struct FastPlan {
+    int kind;             // 0 = codes, 1 = neighbour-code layout, 2 = node-id-range shards
+    uint32_t rounds;      // slots per thread
+    uint32_t list_regs;   // short form: list registers per lane; 0 = long form
+    uint32_t pool_len;    // short form: entries of the tail's pool
+    bool may_mark;        // short form: the long form is launched behind it for the queries it marks
+    uint32_t list_len;
+    bool two_lists, late;
+    uint32_t smem, long_smem;
+};
+bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan);
+cudaError_t LaunchFast(BeamArgs a, const FastPlan& plan, uint64_t num_queries, cudaStream_t stream);
+uint32_t FastBlocksPerSm(const FastPlan& plan);
+// The PQ pivots laid out for the in-kernel table build: dim * 256 floats.
+bool CanPackPivots(uint32_t M, uint32_t dim);
+cudaError_t LaunchPackPivots(const float* col_major, uint32_t M, uint32_t dim, float* out, cudaStream_t stream);
+
 cudaError_t LaunchLutBuild(const float* tables_col_major, const float* centroid,
                            const uint32_t* chunk_offsets, uint32_t dim, uint32_t M,
                            const void* queries, uint32_t query_kind, uint64_t Q, float* out,
