@@ -287,7 +287,10 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
     unsigned long long* fkey = reinterpret_cast<unsigned long long*>(smem_raw + lay.fkey);
     unsigned long long* pool = reinterpret_cast<unsigned long long*>(smem_raw + lay.pool);
     __shared__ unsigned long long s_thr;       // last key of the list; a new key behind it cannot enter
-    __shared__ uint32_t s_count;               // new keys of the push | passing slots << 16
+    __shared__ __align__(16) uint32_t s_count[4];   // per slot warp: new keys of the push | passing slots << 16
+    __shared__ __align__(16) unsigned long long s_sort[32];
+    __shared__ unsigned long long s_open_key[32], s_end[2];   // of the list warp: its first unexpanded keys and their ranks; ranks L - 1, L - 2
+    __shared__ uint32_t s_open_rank[32];
     __shared__ uint32_t s_pool_n, s_tail_thr, s_fail, s_range[2];
     __shared__ uint32_t s_nsel, s_cut;         // nodes selected (0 ends the search); the pool is to be cut
     __shared__ uint32_t s_node[TANN_MAX_SEARCH_WIDTH];
@@ -301,7 +304,7 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
 
     if (warp < 4) {
         // ================================================ slot warps ========================================================
-        const uint64_t N = a.ix.num_nodes;
+        const uint32_t N = (uint32_t)a.ix.num_nodes;   // below 2^30 (checked by the launcher)
         const uint32_t lt = (1u << lane) - 1u;
         uint32_t my_k[kR], my_j[kR];          // this thread's slots: node my_k, neighbour my_j
         uint32_t id[kR], words[kR][kM / 4];
@@ -338,6 +341,8 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 for (int r = 0; r < kR; ++r)
                     if (id[r] < N) LoadCodesXor<kM>(Row<kOneShard>(a.ix.codes, id[r], kM), lane, words[r]);
             }
+            // (a threshold from before the last merge is an upper bound: the list warp sorts out the rest)
+            const unsigned long long thr = *reinterpret_cast<volatile unsigned long long*>(&s_thr);
             BloomBits bits[kR];
             bool pass[kR];
             unsigned long long key[kR];
@@ -346,7 +351,7 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 bits[r] = BloomPositions(id[r]);
                 pass[r] = id[r] < N;
                 // an id that is neither the padding value nor a node of the index is skipped and reported
-                if (id[r] != kInvalid && !pass[r] && a.status != nullptr) atomicOr(a.status, TANN_STATUS_BEAM_ID_RANGE);
+                if (!pass[r] && id[r] != kInvalid && a.status != nullptr) atomicOr(a.status, TANN_STATUS_BEAM_ID_RANGE);
             }
             if (hash_iter == 0 && push != 0) BlockSync();   // the list warp has rebuilt the filter
             pass[0] = pass[0] && !BloomTest(bits[0], bloom);
@@ -368,39 +373,29 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 key[r] = ((unsigned long long)OrderedBits(AdcXor<kM>(smem_raw, words[r], offs)) << 32) | (id[r] << 2);
             }
             // ---- which new keys go to the list, which into the tail ----------------------------------------------------------
-            // (a threshold from before the last merge is an upper bound: the list warp sorts out the rest)
-            const unsigned long long thr = *reinterpret_cast<volatile unsigned long long*>(&s_thr);
-            uint32_t to_list[kR], to_tail[kR], mine = 0, mine_tail = 0;
+            uint32_t to_tail[kR], mine = 0, mine_tail = 0;
+            unsigned long long* segment = fkey + (push & 1u) * kFresh + warp * (32u * kR);
 #pragma unroll
             for (int r = 0; r < kR; ++r) {
                 const bool surv = pass[r] && key[r] < thr;
-                to_list[r] = __ballot_sync(kFull, surv);
-                mine += __popc(to_list[r]) + (__popc(__ballot_sync(kFull, pass[r])) << 16);
+                const uint32_t b = __ballot_sync(kFull, surv);
+                if (surv) segment[(mine & 0xffffu) + __popc(b & lt)] = key[r];
+                mine += __popc(b) + (__popc(__ballot_sync(kFull, pass[r])) << 16);
                 to_tail[r] = 0;
                 if (tail) {
                     to_tail[r] = __ballot_sync(kFull, pass[r] && !surv && (uint32_t)(key[r] >> 32) <= s_tail_thr);
                     mine_tail += __popc(to_tail[r]);
                 }
             }
-            uint32_t base = 0, base_tail = 0;
-            if (lane == 0) {
-                if (mine != 0) base = atomicAdd(&s_count, mine);
-                if (tail && mine_tail != 0) base_tail = atomicAdd(&s_pool_n, mine_tail);
-            }
-            base = __shfl_sync(kFull, base, 0) & 0xffffu;
-            unsigned long long* fresh = fkey + (push & 1u) * kFresh;
-#pragma unroll
-            for (int r = 0; r < kR; ++r) {
-                if ((to_list[r] >> lane) & 1u) fresh[base + (r == 1 ? __popc(to_list[0]) : 0u) + __popc(to_list[r] & lt)] = key[r];
-            }
-            if (tail) {
-                base_tail = __shfl_sync(kFull, base_tail, 0);
+            if (lane == 0) s_count[warp] = mine;
+            if (tail && mine_tail != 0) {
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&s_pool_n, mine_tail);
+                at = __shfl_sync(kFull, at, 0);
 #pragma unroll
                 for (int r = 0; r < kR; ++r) {
-                    if ((to_tail[r] >> lane) & 1u) {
-                        const uint32_t at = base_tail + (r == 1 ? __popc(to_tail[0]) : 0u) + __popc(to_tail[r] & lt);
-                        if (at < a.pool_len) pool[at] = key[r];   // (an overflow is seen by the list warp)
-                    }
+                    const uint32_t mine_at = at + (r == 1 ? __popc(to_tail[0]) : 0u) + __popc(to_tail[r] & lt);
+                    if (((to_tail[r] >> lane) & 1u) && mine_at < a.pool_len) pool[mine_at] = key[r];   // (an overflow is seen by the list warp)
                 }
             }
             BlockSync();
@@ -487,109 +482,167 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
         for (int r = 0; r < kList; ++r) list[r] = kNoKey;
         if (lane == 0) {
             s_thr = kNoKey;
-            s_count = 0; s_pool_n = 0; s_tail_thr = 0xffffffffu; s_fail = 0; s_nsel = 0; s_cut = 0;
+            s_pool_n = 0; s_tail_thr = 0xffffffffu; s_fail = 0; s_nsel = 0; s_cut = 0;
         }
         uint32_t valid = 0, visited = 0, expanded = 0, iterations = 0, first_full = 0xffffffffu, hash_iter = 0, fail = 0;
-        // lane x: the x-th unexpanded entry of the list, and its rank
-        unsigned long long un_key = kNoKey;
-        uint32_t un_pos = 0;
+        // The first unexpanded entries of the list and their ranks: for W <= 2 the same in every lane, else lane x holds the
+        // x-th one (in un_key_0). And the keys of ranks L - 1 and L - 2: a new key below them lies within the first L ranks,
+        // alone or behind one other new key.
+        unsigned long long un_key_0 = kNoKey, un_key_1 = kNoKey, at_end_0 = kNoKey, at_end_1 = L > 1 ? kNoKey : 0ull;
+        uint32_t un_pos_0 = 0, un_pos_1 = 0;
+        constexpr uint32_t kSeg = 32u * kR;
         BlockSync();
         for (uint32_t push = 0; entry_pushes != 0; ++push) {
             BlockSync();   // the push's new keys are there
-            unsigned long long* fresh = fkey + (push & 1u) * kFresh;
-            const uint32_t counts = s_count, n = counts & 0xffffu, fv = counts >> 16;
+            const unsigned long long* fresh = fkey + (push & 1u) * kFresh;
+            const uint4 c4 = *reinterpret_cast<const uint4*>(s_count);
+            const uint32_t counts = c4.x + c4.y + c4.z + c4.w, n = counts & 0xffffu, fv = counts >> 16;
+            const uint32_t e0 = c4.x & 0xffffu, e1 = e0 + (c4.y & 0xffffu), e2 = e1 + (c4.z & 0xffffu);
+            // new key i: the warps' segments one behind the other
+            const auto new_key = [&](uint32_t i) {
+                const uint32_t at = i + (i >= e2 ? 3u * kSeg - e2 : (i >= e1 ? 2u * kSeg - e1 : (i >= e0 ? kSeg - e0 : 0u)));
+                return i < n ? fresh[at] : kNoKey;
+            };
             const uint32_t pool_n = tail ? s_pool_n : 0u;
-            const uint32_t nv = (uint32_t)min((uint64_t)C, (uint64_t)valid + fv);
-            if (first_full == 0xffffffffu && nv >= L) first_full = push < entry_pushes ? 0u : iterations;
-            visited += fv;
-            valid = nv;
             const bool more = push + 1 < entry_pushes;   // the next push takes entries again
             // ---- selection -----------------------------------------------------------------------------------------------------
-            unsigned long long k0 = lane < n ? fresh[lane] : kNoKey;   // new keys [0, 32)
+            const unsigned long long k0 = new_key(lane);
             uint32_t nsel = 0, list_end = 0;
-            unsigned long long last_pick = 0;
+            unsigned long long done_key = 0ull;   // the largest new key selected (the smaller ones all are) ...
+            uint32_t done = 0;                    // ... how many copies of it ...
+            unsigned long long last_old = 0ull;   // ... and the last list entry selected
             if (!more && expanded < a.p.max_expansions) {
-                unsigned long long least = k0;
-                uint32_t at = lane, pick = 0, un_taken = 0, new_picks = 0;
+                unsigned long long m0 = k0, m1 = kNoKey;   // the two least of this lane's keys
 #pragma unroll 1
-                for (uint32_t i = 32u + lane; i < n; i += 32u) {
-                    const unsigned long long k = fresh[i];
-                    if (k < least) { least = k; at = i; }
+                for (uint32_t i = 32u; i < n; i += 32u) {
+                    const unsigned long long k = new_key(i + lane);
+                    m1 = k < m0 ? m0 : (k < m1 ? k : m1);
+                    m0 = k < m0 ? k : m0;
                 }
-                unsigned long long s_min = n != 0 ? WarpMinKey(least) : kNoKey;
-#pragma unroll 1
-                while (nsel < W) {
-                    const unsigned long long u = __shfl_sync(kFull, un_key, un_taken);
-                    if (s_min < u) {
-                        // inside the first L ranks?
-                        uint32_t below = new_picks;
-#pragma unroll
-                        for (int r = 0; r < kList; ++r) below += __popc(__ballot_sync(kFull, list[r] < s_min));
-                        if (below >= L) break;
-                        if (lane == nsel) pick = (uint32_t)s_min >> 2;
-                        last_pick = s_min;
-                        ++nsel;
-                        ++new_picks;
-                        const uint32_t owner = __ffs(__ballot_sync(kFull, least == s_min)) - 1u;
-                        if (lane == owner) {   // selected: expanded from now on
-                            if (at < 32u) k0 |= kExpanded; else fresh[at] = least | kExpanded;
-                            least = kNoKey;
-                            if (n > 32u) {
-                                if (lane < n && (k0 & 3u) == kNew) { least = k0; at = lane; }
-#pragma unroll 1
-                                for (uint32_t i = 32u + lane; i < n; i += 32u) {
-                                    const unsigned long long k = fresh[i];
-                                    if ((k & 3u) == kNew && k < least) { least = k; at = i; }
+                const unsigned long long s0 = WarpMinKey(m0);
+                if (W <= 2) {
+                    const uint32_t holders = __ballot_sync(kFull, m0 == s0);
+                    const bool owner = m0 == s0 && (holders & ((1u << lane) - 1u)) == 0u;
+                    const unsigned long long s1 = WarpMinKey(owner ? m1 : m0);
+                    const bool new_first = s0 < un_key_0;
+                    if (new_first ? s0 < at_end_0 : un_key_0 < kNoKey) {
+                        nsel = 1;
+                        uint32_t id0, id1 = 0;
+                        if (new_first) { done_key = s0; done = 1; id0 = (uint32_t)s0 >> 2; }
+                        else { last_old = un_key_0; list_end = un_pos_0 + 1u; id0 = (uint32_t)last_old >> 2; }
+                        if (W == 2) {
+                            const unsigned long long s = new_first ? s1 : s0, u = new_first ? un_key_0 : un_key_1;
+                            const uint32_t u_pos = new_first ? un_pos_0 + 1u : un_pos_1;
+                            if (s < u) {
+                                if (s < (new_first ? at_end_1 : at_end_0)) {
+                                    nsel = 2;
+                                    id1 = (uint32_t)s >> 2;
+                                    done = s == done_key ? 2u : 1u;
+                                    done_key = s;
                                 }
+                            } else if (u < kNoKey && u_pos < L) {
+                                nsel = 2;
+                                id1 = (uint32_t)u >> 2;
+                                last_old = u;
+                                list_end = (new_first ? un_pos_0 : un_pos_1) + 1u;
                             }
                         }
-                        if (nsel < W) s_min = WarpMinKey(least);
-                    } else if (u < kNoKey) {
-                        const uint32_t pos = __shfl_sync(kFull, un_pos, un_taken);
-                        if (pos + new_picks >= L) break;
-                        if (lane == nsel) pick = (uint32_t)u >> 2;
-                        last_pick = u;
-                        list_end = pos + 1u;
-                        ++un_taken;
-                        ++nsel;
-                    } else {
-                        break;
+                        if (lane < 2) s_node[lane] = lane == 0 ? id0 : id1;
                     }
+                } else {
+                    // general widths, one selection after the other
+                    unsigned long long s_min = s0;
+                    uint32_t un_taken = 0, pick = 0, new_picks = 0;
+#pragma unroll 1
+                    while (nsel < W) {
+                        const unsigned long long u = __shfl_sync(kFull, un_key_0, un_taken);
+                        if (s_min < u) {
+                            uint32_t below = new_picks;
+#pragma unroll
+                            for (int r = 0; r < kList; ++r) below += __popc(__ballot_sync(kFull, list[r] < s_min));
+                            if (below >= L) break;
+                            if (lane == nsel) pick = (uint32_t)s_min >> 2;
+                            done = s_min == done_key ? done + 1u : 1u;
+                            done_key = s_min;
+                            ++nsel;
+                            ++new_picks;
+                            // the next one: another copy of the same key, or the least above it
+                            uint32_t copies = 0;
+                            unsigned long long least = kNoKey;
+#pragma unroll 1
+                            for (uint32_t i = 0; i < n; i += 32u) {
+                                const unsigned long long k = new_key(i + lane);
+                                copies += __popc(__ballot_sync(kFull, k == done_key));
+                                if (k > done_key && k < least) least = k;
+                            }
+                            s_min = copies > done ? done_key : WarpMinKey(least);
+                        } else if (u < kNoKey) {
+                            const uint32_t pos = __shfl_sync(kFull, un_pos_0, un_taken);
+                            if (pos + new_picks >= L) break;
+                            if (lane == nsel) pick = (uint32_t)u >> 2;
+                            last_old = u;
+                            list_end = pos + 1u;
+                            ++un_taken;
+                            ++nsel;
+                        } else {
+                            break;
+                        }
+                    }
+                    if (lane < nsel) s_node[lane] = pick;
                 }
-                if (lane < nsel) s_node[lane] = pick;
-                if (nsel != 0) ++iterations;
-                expanded += nsel;
             }
             // the pool must take this push's displaced entries and the next push's tail keys
             const bool cut = tail && pool_n + n + kFresh > a.pool_len;
             if (lane == 0) {
                 s_nsel = nsel;
-                s_count = 0;
-                s_cut = cut ? 1u : 0u;
+                if (tail) s_cut = cut ? 1u : 0u;
             }
-            if (tail && pool_n > a.pool_len) fail = 1;
             BlockSync();   // the selection is there
             const bool last_push = !more && nsel == 0;
+            if (tail && pool_n > a.pool_len) fail = 1;
             if (cut && !last_push) BlockSync();
             // ---- merge, behind the next push's loads ------------------------------------------------------------------------------
-            if (list_end != 0u) {   // every unexpanded entry up to there was selected
+            const uint32_t nv = (uint32_t)min((uint64_t)C, (uint64_t)valid + fv);
+            if (first_full == 0xffffffffu && nv >= L) first_full = push < entry_pushes ? 0u : iterations;
+            visited += fv;
+            valid = nv;
+            iterations += nsel != 0u ? 1u : 0u;
+            expanded += nsel;
+            if (list_end != 0u) {   // every unexpanded entry up to there was selected; a twin of the last one stays behind it
 #pragma unroll
-                for (int r = 0; r < kList; ++r)
+                for (int r = 0; r < kList; ++r) {
                     if (r * 32u + lane < list_end) list[r] = (list[r] & ~3ull) | kExpanded;
+                    else if (((list[r] ^ last_old) >> 2) == 0ull) list[r] = (list[r] & ~3ull) | kTwin;
+                }
             }
-            if (nsel != 0u) {   // a twin of the last selected node that was not selected stays behind it
-#pragma unroll
-                for (int r = 0; r < kList; ++r)
-                    if ((list[r] >> 2) == (last_pick >> 2) && (list[r] & 3u) == kNew) list[r] |= kTwin;
-                if ((k0 >> 2) == (last_pick >> 2) && (k0 & 3u) == kNew) k0 |= kTwin;
-#pragma unroll 1
-                for (uint32_t i = 32u + lane; i < n; i += 32u)
-                    if ((fresh[i] >> 2) == (last_pick >> 2) && (fresh[i] & 3u) == kNew) fresh[i] |= kTwin;
-            }
+            uint32_t copies = 0;
 #pragma unroll 1
             for (uint32_t c = 0; c < n; c += 32u) {
-                if (c != 0) k0 = c + lane < n ? fresh[c + lane] : kNoKey;
-                unsigned long long out = MergeIntoList<kList>(list, WarpSortDescending(k0, lane), lane);
+                unsigned long long k = c == 0 ? k0 : new_key(c + lane);
+                if (done != 0u) {
+                    const uint32_t same = __ballot_sync(kFull, k == done_key);
+                    if (k < done_key) k |= kExpanded;
+                    else if (k == done_key) k |= copies + __popc(same & ((1u << lane) - 1u)) < done ? kExpanded : kTwin;
+                    copies += __popc(same);
+                }
+                // descending order by rank counting
+                s_sort[lane] = k;
+                __syncwarp();
+                uint32_t rank = 0;
+                const uint32_t m = min(n - c, 32u);
+#pragma unroll 1
+                for (uint32_t j = 0; j < m; j += 8u) {
+                    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(s_sort + j);
+                    const ulonglong2 a0 = p[0], a1 = p[1], a2 = p[2], a3 = p[3];
+                    rank += (a0.x < k ? 1u : 0u) + (a0.y < k ? 1u : 0u) + (a1.x < k ? 1u : 0u) + (a1.y < k ? 1u : 0u);
+                    rank += (a2.x < k ? 1u : 0u) + (a2.y < k ? 1u : 0u) + (a3.x < k ? 1u : 0u) + (a3.y < k ? 1u : 0u);
+                }
+                rank += __popc(__match_any_sync(kFull, rank) & ((1u << lane) - 1u));   // equal keys: any order
+                __syncwarp();
+                s_sort[31u - rank] = k;
+                __syncwarp();
+                unsigned long long out = MergeIntoList<kList>(list, s_sort[lane], lane);
+                __syncwarp();
                 if (tail) {
                     const uint32_t b = __ballot_sync(kFull, out != kNoKey);
                     if (b != 0u) {
@@ -600,25 +653,20 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                         at += __popc(b & ((1u << lane) - 1u));
                         if (out != kNoKey && at < a.pool_len) pool[at] = out;
                     }
-                } else {
-                    if (cap < 32u * kList) {   // a list shorter than the registers hold
-                        const unsigned long long last = __shfl_sync(kFull, list[0], cap - 1u);
-                        if (C > L && __any_sync(kFull, out != kNoKey && (out >> 2) == (last >> 2) && out != last)) fail = 1;
-                        if (lane >= cap) { out = list[0]; list[0] = kNoKey; }
-                    }
-                    if (C > L) {
-                        // copies of one node across the end of the list, in different states
-                        const uint32_t end = cap - 1u;
-                        const unsigned long long last = __shfl_sync(kFull, list[kList - 1], end & 31u);
-                        if (__any_sync(kFull, out != kNoKey && (out >> 2) == (last >> 2) && out != last)) fail = 1;
-                    }
+                } else if (C > L) {
+                    // copies of one node across the end of the list, in different states
+                    const unsigned long long last = __shfl_sync(kFull, list[kList - 1], (cap - 1u) & 31u);
+                    if (__any_sync(kFull, out != kNoKey && ((out ^ last) >> 2) == 0ull && out != last)) fail = 1;
+                }
+                if (cap < 32u * kList) {   // a list shorter than the registers hold (kList is 1)
+                    const unsigned long long last = __shfl_sync(kFull, list[0], cap - 1u);
+                    const bool beyond = lane >= cap && list[0] != kNoKey;
+                    if (C > L && __any_sync(kFull, beyond && ((list[0] ^ last) >> 2) == 0ull && list[0] != last)) fail = 1;
+                    if (beyond) list[0] = kNoKey;
                 }
             }
             if (last_push) break;
-            if (n != 0) {
-                const unsigned long long last = __shfl_sync(kFull, list[kList - 1], (cap - 1u) & 31u);
-                if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(&s_thr) = last;
-            }
+            if (lane == ((cap - 1u) & 31u)) *reinterpret_cast<volatile unsigned long long*>(&s_thr) = list[kList - 1];
             if (++hash_iter >= 3) {
                 hash_iter = 0;
 #pragma unroll
@@ -626,23 +674,32 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                     if (r * 32u + lane < L && list[r] != kNoKey) BloomAdd((uint32_t)list[r] >> 2, bloom);
                 BlockSync();   // the filter is complete
             }
-            // the first W unexpanded ranks below L
-            {
-                uint32_t found = 0;
-                un_key = kNoKey;
+            // the first unexpanded ranks below L
+            uint32_t open = 0;
 #pragma unroll
-                for (int r = 0; r < kList; ++r) {
-                    uint32_t b = __ballot_sync(kFull, r * 32u + lane < L && list[r] != kNoKey && (list[r] & 3u) != kExpanded);
-#pragma unroll 1
-                    while (b != 0u && found < W) {
-                        const uint32_t src = __ffs(b) - 1u;
-                        const unsigned long long k = __shfl_sync(kFull, list[r], src);
-                        if (lane == found) { un_key = k; un_pos = r * 32u + src; }
-                        b &= b - 1u;
-                        ++found;
-                    }
-                }
+            for (int r = 0; r < kList; ++r) {
+                const uint32_t rank = r * 32u + lane;
+                const bool mine = rank < L && list[r] != kNoKey && ((uint32_t)list[r] & 3u) != kExpanded;
+                const uint32_t b = __ballot_sync(kFull, mine);
+                const uint32_t order = open + __popc(b & ((1u << lane) - 1u));
+                if (mine && order < W) { s_open_key[order] = list[r]; s_open_rank[order] = rank; }
+                if (rank == L - 1u) s_end[0] = list[r];
+                if (rank + 2u == L) s_end[1] = list[r];
+                open += __popc(b);
             }
+            __syncwarp();
+            if (W <= 2) {
+                un_key_0 = open > 0u ? s_open_key[0] : kNoKey;
+                un_pos_0 = s_open_rank[0];
+                un_key_1 = W == 2u && open > 1u ? s_open_key[1] : kNoKey;
+                un_pos_1 = s_open_rank[1];
+                at_end_0 = s_end[0];
+                if (L > 1u) at_end_1 = s_end[1];
+            } else {
+                un_key_0 = lane < open ? s_open_key[lane] : kNoKey;
+                un_pos_0 = s_open_rank[lane];
+            }
+            __syncwarp();
         }
         if (entry_pushes == 0) return;
         // ---- results: the list's ranks -----------------------------------------------------------------------------------------

@@ -12,42 +12,40 @@
 
 namespace tann {
 
-// A row's 16-byte pieces, permuted so that byte b of the result is chunk b ^ lane of its group of 32 (or 16) chunks.
+// The 16-byte pieces of a code row, in the order in which lane `lane` uses them (bit 4 of the lane exchanges the two pieces
+// of a group of 32 chunks).
 template <int kM>
 __device__ __forceinline__ void LoadCodesXor(const uint8_t* row, uint32_t lane, uint32_t (&w)[kM / 4]) {
     const uint4* r4 = reinterpret_cast<const uint4*>(row);
 #pragma unroll
     for (int i = 0; i < kM / 16; ++i) {
-        // lane bit 4 exchanges the two pieces of a group of 32
         const int piece = (i | 1) * 16 < kM ? (int)((uint32_t)i ^ (lane >> 4)) : i;
         const uint4 v = __ldg(r4 + piece);
         w[4 * i + 0] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
     }
 }
+// Bits 2 and 3 of the lane exchange the words of a piece: word j then holds chunks 4 (j ^ lane / 4) + {0..3}.
 template <int kM>
 __device__ __forceinline__ void PermuteXor(uint32_t lane, uint32_t (&w)[kM / 4]) {
     const bool b3 = (lane & 8u) != 0, b2 = (lane & 4u) != 0;
-    const uint32_t sel = 0x3210u ^ ((lane & 3u) * 0x1111u);
 #pragma unroll
     for (int i = 0; i < kM / 16; ++i) {
-        uint32_t a = w[4 * i], b = w[4 * i + 1], c = w[4 * i + 2], d = w[4 * i + 3];
+        const uint32_t a = w[4 * i], b = w[4 * i + 1], c = w[4 * i + 2], d = w[4 * i + 3];
         const uint32_t a1 = b3 ? c : a, c1 = b3 ? a : c, b1 = b3 ? d : b, d1 = b3 ? b : d;
-        a = b2 ? b1 : a1; b = b2 ? a1 : b1; c = b2 ? d1 : c1; d = b2 ? c1 : d1;
-        w[4 * i] = __byte_perm(a, 0, sel); w[4 * i + 1] = __byte_perm(b, 0, sel);
-        w[4 * i + 2] = __byte_perm(c, 0, sel); w[4 * i + 3] = __byte_perm(d, 0, sel);
+        w[4 * i] = b2 ? b1 : a1; w[4 * i + 1] = b2 ? a1 : b1;
+        w[4 * i + 2] = b2 ? d1 : c1; w[4 * i + 3] = b2 ? c1 : d1;
     }
 }
 
-// The table sum of one node. x[k] (k = 0..7) holds, for the words 4 k .. 4 k + 3 of a group, the byte offsets of the
-// chunks in a table row: bytes 0 and 2 of the word in x[2 k'] ... - see LaneOffsets().
+// What a lane needs to turn a byte of a code word into the byte offset of its table entry with one dp4a: step c of a group
+// reads chunk c ^ lane, i.e. byte (c ^ lane) & 3 of the permuted word c / 4, at code * 128 + 4 (c ^ lane).
 struct LaneOffsets {
-    uint32_t even[8], odd[8];   // word j of a group: chunks 4 j + {0, 2} and 4 j + {1, 3}, as two 16-bit byte offsets each
+    uint32_t chunk[32], row[4];
     __device__ __forceinline__ explicit LaneOffsets(uint32_t lane) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            even[j] = (((4u * j + 0u) ^ lane) << 2) | (((4u * j + 2u) ^ lane) << 18);
-            odd[j] = (((4u * j + 1u) ^ lane) << 2) | (((4u * j + 3u) ^ lane) << 18);
-        }
+        for (uint32_t c = 0; c < 32; ++c) chunk[c] = (c ^ lane) << 2;
+#pragma unroll
+        for (uint32_t b = 0; b < 4; ++b) row[b] = 128u << (8u * ((b ^ lane) & 3u));
     }
 };
 template <int kM>
@@ -55,25 +53,16 @@ __device__ __forceinline__ float AdcXor(const unsigned char* lut, const uint32_t
     float total = 0.0f;
 #pragma unroll
     for (int base = 0; base < kM; base += 32) {
-        constexpr bool kDummy = true; (void)kDummy;
         const int n = (kM - base) < 32 ? (kM - base) : 32;
         const unsigned char* t = lut + base * 1024;
         float2 x[16];
 #pragma unroll
-        for (int j = 0; j < n / 4; ++j) {
-            const uint32_t v = w[base / 4 + j];
-            uint32_t e, d;
-            if (n == 32) {
-                e = ((v << 7) & 0x7f807f80u) | o.even[j];
-                d = ((v >> 1) & 0x7f807f80u) | o.odd[j];
-            } else {   // groups of 16 chunks: rows of 64 bytes, lanes l and l + 16 read the same chunk
-                e = ((v << 6) & 0x3fc03fc0u) | (o.even[j] & 0x003c003cu);
-                d = ((v >> 2) & 0x3fc03fc0u) | (o.odd[j] & 0x003c003cu);
-            }
-            x[2 * j].x = *reinterpret_cast<const float*>(t + (e & 0xffffu));
-            x[2 * j].y = *reinterpret_cast<const float*>(t + (d & 0xffffu));
-            x[2 * j + 1].x = *reinterpret_cast<const float*>(t + (e >> 16));
-            x[2 * j + 1].y = *reinterpret_cast<const float*>(t + (d >> 16));
+        for (int c = 0; c < n; ++c) {
+            // groups of 16 chunks: rows of 64 bytes, lanes l and l + 16 read the same chunk
+            const uint32_t at = n == 32 ? __dp4a(w[(base + c) / 4], o.row[c & 3], o.chunk[c])
+                                        : __dp4a(w[(base + c) / 4], o.row[c & 3] >> 1, o.chunk[c] & 0x3cu);
+            const float v = *reinterpret_cast<const float*>(t + at);
+            if ((c & 1) == 0) x[c / 2].x = v; else x[c / 2].y = v;
         }
 #pragma unroll
         for (int off = 8; off >= 1; off >>= 1) {
