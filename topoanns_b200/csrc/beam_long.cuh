@@ -54,7 +54,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
     uint32_t* taken = reinterpret_cast<uint32_t*>(smem_raw + lay.words);
     uint32_t* unexp = taken + kTakenWords;
     __shared__ uint32_t s_count[2];       // new keys | passing slots << 16 of a push, two pushes in turn
-    __shared__ uint32_t s_flag;
+    __shared__ uint32_t s_flag, s_marks[kBeamThreads / 32];
     __shared__ __align__(16) LongPicks picks;
     __shared__ BeamCtl ctl;
     const LaneOffsets offs(lane);
@@ -66,33 +66,33 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
         my_k[r] = (r * kBeamThreads + tid) / deg;
         my_j[r] = r * kBeamThreads + tid - my_k[r] * deg;
     }
-    for (uint64_t q = blockIdx.x; q < a.num_queries; q += gridDim.x) {
-    if (a.only_marked != 0u && a.out_stats[q * 8 + 6] == 0u) continue;
+    // Marked queries are few: the block looks at the marks of 128 of its queries at a time (one dependent load per query
+    // took 32 us for 10 k queries, the launch now takes 13).
+    const uint32_t group = a.only_marked != 0u ? (uint32_t)kBeamThreads : 1u;
+    for (uint64_t first = blockIdx.x; first < a.num_queries; first += (uint64_t)gridDim.x * group) {
+    if (a.only_marked != 0u) {
+        const uint64_t mine = first + (uint64_t)tid * gridDim.x;
+        const uint32_t marks = __ballot_sync(kFull, mine < a.num_queries && a.out_stats[mine * 8 + 6] != 0u);
+        __syncthreads();   // the marks before are worked off
+        if (lane == 0) s_marks[warp] = marks;
+        __syncthreads();
+    }
+    for (uint32_t g = 0; g < group; ++g) {
+    if (a.only_marked != 0u && ((s_marks[g >> 5] >> (g & 31u)) & 1u) == 0u) continue;
+    const uint64_t q = first + (uint64_t)g * gridDim.x;
     const uint32_t entry_begin = a.entry_offsets[q];
     const uint32_t num_entries = a.entry_offsets[q + 1] - entry_begin;
 
     // ---- the query's table ---------------------------------------------------------------------------------------------
-    {
-        const uint32_t d = a.ix.dim;
-        __syncthreads();   // the query before is done
-        float* sq = reinterpret_cast<float*>(bloom);   // dim <= kBloomWords (checked by the launcher)
-        const float* given = a.lut != nullptr ? a.lut + q * (uint64_t)kM * kCentroids : nullptr;
-        if (given == nullptr)   // src/search/pq_query_tables.cu:33-52
-            for (uint32_t i = tid; i < d; i += kBeamThreads)
-                sq[i] = LoadAsFloat<float>(a.queries, a.query_kind, q * d + i) - __ldg(a.ix.pq_centroid + i);
-        __syncthreads();
-        if (given == nullptr && a.pivots_packed != nullptr && d == 2 * kM) TableFromPacked<kM, 2>(lut, sq, a.pivots_packed, tid);
-        else if (given == nullptr && a.pivots_packed != nullptr && d == 4 * kM) TableFromPacked<kM, 4>(lut, sq, a.pivots_packed, tid);
-        else if (given == nullptr && a.pivots_packed != nullptr && d == 8 * kM) TableFromPacked<kM, 8>(lut, sq, a.pivots_packed, tid);
-        else TableFromColumns<kM>(lut, sq, a, given, tid);
-    }
+    __syncthreads();   // the query before is done
+    // dim <= kBloomWords (checked by the launcher)
+    BuildTable<kM>(lut, reinterpret_cast<float*>(bloom), a, q, tid, [] { __syncthreads(); });
 
     const uint32_t list_len = a.list_len;
     const bool two_lists = a.two_lists != 0;
     {
         unsigned long long* cur = reinterpret_cast<unsigned long long*>(smem_raw + lay.list);
         unsigned long long* nxt = two_lists ? reinterpret_cast<unsigned long long*>(smem_raw + lay.other) : cur;
-        __syncthreads();
         for (uint32_t i = tid; i < kBloomWords / 4; i += kBeamThreads) reinterpret_cast<uint4*>(bloom)[i] = make_uint4(0, 0, 0, 0);
         if (tid < kTakenWords + 32) taken[tid] = 0u;
         if (tid < 2) s_count[tid] = 0;
@@ -452,6 +452,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
             st[0] = visited; st[1] = expanded; st[2] = 0; st[3] = iterations;
             st[4] = valid; st[5] = first_full; st[6] = 0; st[7] = 0;
         }
+    }
     }
     }
 }

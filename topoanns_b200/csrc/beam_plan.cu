@@ -61,8 +61,8 @@ bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan) 
     plan->list_regs = 0;
     plan->pool_len = 0;
     plan->may_mark = false;
-    if (L > 128 || late || ix.num_nodes > 0x3fffffffull) return true;
-    const uint32_t regs = L <= 32 ? 1u : (L <= 64 ? 2u : 4u);
+    if (L > 256 || late || ix.num_nodes > 0x3fffffffull) return true;
+    const uint32_t regs = L <= 32 ? 1u : (L <= 64 ? 2u : (L <= 128 ? 4u : 8u));
     if (C > 32 * regs) {
         // room for the ranks behind the list, the keys of two pushes and some slack for the cut
         const uint32_t want = C - 32 * regs + 64 + 256 * plan->rounds, most = kSlotThreads * kTailPer;

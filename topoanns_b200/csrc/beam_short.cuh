@@ -315,21 +315,8 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
             my_j[r] = s - my_k[r] * deg;
             id[r] = (s < slots && s < num_entries) ? __ldg(a.entry_ids + entry_begin + s) : kInvalid;
         }
-        {
-            const uint32_t d = a.ix.dim;
-            float* lut = reinterpret_cast<float*>(smem_raw);
-            float* sq = reinterpret_cast<float*>(bloom);   // dim <= kBloomWords (checked by the launcher)
-            const float* given = a.lut != nullptr ? a.lut + q * (uint64_t)kM * kCentroids : nullptr;
-            if (given == nullptr)   // src/search/pq_query_tables.cu:33-52
-                for (uint32_t i = tid; i < d; i += kSlotThreads)
-                    sq[i] = LoadAsFloat<float>(a.queries, a.query_kind, q * d + i) - __ldg(a.ix.pq_centroid + i);
-            SlotSync();
-            if (given == nullptr && a.pivots_packed != nullptr && d == 2 * kM) TableFromPacked<kM, 2>(lut, sq, a.pivots_packed, tid);
-            else if (given == nullptr && a.pivots_packed != nullptr && d == 4 * kM) TableFromPacked<kM, 4>(lut, sq, a.pivots_packed, tid);
-            else if (given == nullptr && a.pivots_packed != nullptr && d == 8 * kM) TableFromPacked<kM, 8>(lut, sq, a.pivots_packed, tid);
-            else TableFromColumns<kM>(lut, sq, a, given, tid);
-            SlotSync();
-        }
+        // dim <= kBloomWords (checked by the launcher)
+        BuildTable<kM>(reinterpret_cast<float*>(smem_raw), reinterpret_cast<float*>(bloom), a, q, tid, SlotSync);
         for (uint32_t i = tid; i < kBloomWords / 4; i += kSlotThreads) reinterpret_cast<uint4*>(bloom)[i] = make_uint4(0, 0, 0, 0);
         const LaneOffsets offs(lane);
         BlockSync();

@@ -124,6 +124,15 @@ __device__ __forceinline__ void TableFromPacked(float* lut, const float* sq, con
         }
     }
 }
+// The packed layout is for chunks of one width. Every warp checks all chunks, so that a block decides as one.
+template <int kM>
+__device__ __forceinline__ bool EqualChunks(const uint32_t* offsets, uint32_t dim, uint32_t lane) {
+    bool equal = dim % kM == 0;
+#pragma unroll
+    for (uint32_t m = 0; m <= kM; m += 32)
+        if (m + lane <= kM) equal = equal && __ldg(offsets + m + lane) == (m + lane) * (dim / kM);
+    return __all_sync(kFull, equal);
+}
 // From the column-major pivots (any chunk widths), or copied from a caller's [M][256] table.
 template <int kM>
 __device__ __forceinline__ void TableFromColumns(float* lut, const float* sq, const BeamArgs& a, const float* given, uint32_t tid) {
@@ -158,6 +167,22 @@ __device__ __forceinline__ void TableFromColumns(float* lut, const float* sq, co
             t[(c0 + 3) * width] = acc.w;
         }
     }
+}
+
+// Table of query q (tid: 0 to 127; sq: room for the query's values); `sync` is a barrier of these 128 threads.
+template <int kM, typename Sync>
+__device__ __forceinline__ void BuildTable(float* lut, float* sq, const BeamArgs& a, uint64_t q, uint32_t tid, Sync sync) {
+    const uint32_t d = a.ix.dim;
+    const float* given = a.lut != nullptr ? a.lut + q * (uint64_t)kM * kCentroids : nullptr;
+    const bool packed = a.pivots_packed != nullptr && EqualChunks<kM>(a.ix.pq_chunk_offsets, d, tid & 31);
+    if (given == nullptr)   // src/search/pq_query_tables.cu:33-52
+        for (uint32_t i = tid; i < d; i += 128) sq[i] = LoadAsFloat<float>(a.queries, a.query_kind, q * d + i) - __ldg(a.ix.pq_centroid + i);
+    sync();
+    if (packed && d == 2 * kM) TableFromPacked<kM, 2>(lut, sq, a.pivots_packed, tid);
+    else if (packed && d == 4 * kM) TableFromPacked<kM, 4>(lut, sq, a.pivots_packed, tid);
+    else if (packed && d == 8 * kM) TableFromPacked<kM, 8>(lut, sq, a.pivots_packed, tid);
+    else TableFromColumns<kM>(lut, sq, a, given, tid);
+    sync();
 }
 
 // Smallest key of a warp (all lanes call; every lane returns it).

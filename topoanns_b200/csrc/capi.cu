@@ -181,13 +181,11 @@ TannStatus tann_lut_build(const float* tables_col_major, const float* centroid,
     return TANN_OK;
 }
 
-// pivots_packed: the index's pivots as LaunchPackPivots lays them out, or nullptr.
+// pivots_room: room for the index's pivots as LaunchPackPivots lays them out, or nullptr.
 static TannStatus BeamSearch(const TannIndexView* index, const TannBeamParams* params, const float* lut,
-                             const float* pivots_packed,
-                             const void* queries, uint32_t query_kind, uint64_t num_queries,
-                            const uint32_t* entry_offsets, const uint32_t* entry_ids,
-                            void* out_candidates, uint32_t* out_stats, uint32_t* status,
-                            tann_stream_t stream) {
+                             float* pivots_room, const void* queries, uint32_t query_kind, uint64_t num_queries,
+                             const uint32_t* entry_offsets, const uint32_t* entry_ids, void* out_candidates,
+                             uint32_t* out_stats, uint32_t* status, tann_stream_t stream) {
     TannStatus st = CheckBeam(index, params);
     if (st != TANN_OK) return st;
     if (num_queries == 0) return TANN_OK;
@@ -230,8 +228,13 @@ static TannStatus BeamSearch(const TannIndexView* index, const TannBeamParams* p
     a.out_cand = static_cast<tann::Cand*>(out_candidates);
     a.out_stats = out_stats;
     a.status = status;
-    a.pivots_packed = pivots_packed;
     if (plan.fast_form) {
+        // Laid out on each call (the caller may have changed the index's tables since the last one): 2.2 us for 128 x 256
+        // pivots, and one query's table takes 3 us from there against 22 us from the columns.
+        if (pivots_room != nullptr && lut == nullptr) {
+            TANN_CUDA(tann::LaunchPackPivots(index->pq_tables_col_major, index->num_chunks, index->dim, pivots_room, (cudaStream_t)stream));
+            a.pivots_packed = pivots_room;
+        }
         TANN_CUDA(tann::LaunchFast(a, plan.fast, num_queries, (cudaStream_t)stream));
         return TANN_OK;
     }
@@ -699,7 +702,7 @@ struct TannSearcher {
     unsigned long long* d_counts;
     uint32_t* d_fixed_entries;   // max_entries ids: the fixed entry list before it is expanded per query
     uint32_t* d_status;          // TANN_STATUS_* bits of the last run
-    float* d_pivots;             // the PQ pivots laid out for the in-kernel table build (nullptr: other chunk shapes)
+    float* d_pivots;             // room for the PQ pivots laid out for the in-kernel table build (nullptr: other chunk shapes)
     uint32_t* h_status;
     // pinned staging
     // a batch that tann_searcher_submit enqueued and tann_searcher_wait has not collected yet
@@ -769,19 +772,7 @@ TannStatus tann_searcher_create(const TannIndexView* index, uint64_t max_queries
     dev((void**)&s->d_counts, 16);
     dev((void**)&s->d_fixed_entries, (size_t)max_entries_per_query * 4);
     dev((void**)&s->d_status, 16);
-    bool equal_chunks = false;   // the packed layout is for chunks of one width
-    if (e == cudaSuccess && index->pq_tables_col_major != nullptr && index->pq_chunk_offsets != nullptr &&
-        tann::CanPackPivots(index->num_chunks, index->dim)) {
-        std::vector<uint32_t> offs(index->num_chunks + 1);
-        e = cudaMemcpy(offs.data(), index->pq_chunk_offsets, offs.size() * 4, cudaMemcpyDefault);
-        equal_chunks = e == cudaSuccess;
-        for (size_t m = 0; m < offs.size(); ++m) equal_chunks = equal_chunks && offs[m] == m * (index->dim / index->num_chunks);
-    }
-    if (equal_chunks) {
-        dev((void**)&s->d_pivots, d * 1024);
-        if (e == cudaSuccess) e = tann::LaunchPackPivots(index->pq_tables_col_major, index->num_chunks, index->dim, s->d_pivots, nullptr);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    }
+    if (tann::CanPackPivots(index->num_chunks, index->dim)) dev((void**)&s->d_pivots, d * 1024);
     host((void**)&s->h_status, 16);
     host(&s->h_queries, Q * d * 4);
     host((void**)&s->h_topk_ids, Q * max_top_n * 4);
