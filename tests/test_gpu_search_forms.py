@@ -1,0 +1,75 @@
+"""The forms of the beam search and of the pq2 refine that a call is sent to by its sizes, at the edges of their ranges."""
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from topoanns_b200 import search
+
+from gpu_support import assert_candidates_equal, device_index, fixed_entries, np_u32, small_index
+
+pytestmark = pytest.mark.gpu
+
+
+def _index(chunks):
+    if chunks == 32:
+        return small_index()
+    if chunks == 48:
+        return small_index(name="cfg3", num_nodes=12000, components=60, num_queries=128)
+    return small_index(name="cfg5", num_nodes=6000, components=30, num_queries=64)
+
+
+# top_l on both sides of each list width of the register form (32, 64, 128, 256 ranks) and beyond it; capacities from the list
+# itself to one that keeps a long unsorted tail; steps of up to 128 and up to 256 slots
+@pytest.mark.parametrize("chunks", [32, 48, 96])
+@pytest.mark.parametrize("top_l,width,top_n", [(1, 1, 1), (5, 2, 5), (16, 2, 192), (32, 2, 32), (33, 1, 33), (64, 3, 300), (65, 2, 65),
+                                               (100, 4, 75), (128, 2, 512), (129, 2, 129), (200, 3, 300), (256, 2, 256), (257, 2, 64)])
+def test_beam_search_at_the_edges_of_the_list_widths(chunks, top_l, width, top_n):
+    s, host = _index(chunks)
+    width = min(width, 256 // host["adjacency"].shape[1])
+    q = s.queries.cuda().contiguous()
+    rng = np.random.default_rng(top_l)
+    entries = np.concatenate([[s.medoid], rng.choice(host["codes"].shape[0], 149, replace=False)])
+    eo, ei = fixed_entries(q.shape[0], entries.tolist())
+    p = search.TopologySearchParams(top_k=1, top_l=top_l, search_width=width, max_expansions=2048)
+    cap = p.capacity(top_n)
+    want, want_stats = None, None
+    for layout in ("plain", "neighbor_codes"):
+        ix = device_index(s)
+        lut = search.lut_build(ix, q)
+        if want is None:
+            want, want_stats = orc.beam_search(host["adjacency"], host["codes"], lut.cpu().numpy(), np_u32(eo), np_u32(ei),
+                                               top_l=top_l, search_width=width, max_expansions=2048, capacity=cap)
+        if layout == "neighbor_codes":
+            ix = search.inline_neighbor_codes(ix)
+        cand, stats = search.beam_search(ix, p, eo, ei, queries=q, capacity=cap)
+        assert_candidates_equal(cand, stats, want, want_stats)
+
+
+@pytest.mark.parametrize("top_l", [16, 33, 100, 256])
+@pytest.mark.parametrize("batch", [100, 700])
+def test_pq2_refine_inside_the_searcher_matches_the_table_form(top_l, batch):
+    """A searcher refines without tables, small batches by one block per query and larger ones with the pivots in shared memory;
+    the separate entry point reads tables. The sums are the same operations in the same order: equal bits."""
+    s, host = small_index(name="cfg3", num_nodes=12000, components=60, num_queries=128)
+    ix = device_index(s)
+    q = s.queries.cuda().repeat(6, 1)[:batch].contiguous()
+    t2, c2 = s.pq2_tables.cuda().float().contiguous(), s.pq2_centroid.cuda().float().contiguous()
+    cross = search.pq2_cross_terms(ix.pq_chunk_offsets, s.pq_tables.cuda().float().contiguous(), ix.pq_centroid, t2, c2)
+    p2 = search.Pq2Resources(codes=s.pq2_codes.cuda().contiguous(), tables_col_major=t2.t().contiguous(), centroid=c2,
+                             chunk_offsets=ix.pq_chunk_offsets, error_bounds=s.pq2_error_bounds.cuda().contiguous(),
+                             cross_terms=cross)
+    top_n = min(top_l, 64)
+    tp = search.TopologySearchParams(top_k=10, top_l=top_l, search_width=2, max_expansions=2048)
+    rp = search.RerankExactParams(top_k=10, top_n=top_n, rank_tile_size=16, use_pq2_bound_filter=True)
+    eo, ei = fixed_entries(batch, [s.medoid])
+    cand, stats = search.beam_search(ix, tp, eo, ei, queries=q, capacity=tp.capacity(top_n))
+    lut2 = search.lut_build(ix, q, tables_col_major=p2.tables_col_major, centroid=c2)
+    refined = search.pq2_refine(cand, stats, top_l, p2.codes, lut2, base_codes=ix.codes, cross_terms=cross)
+    d, i, _, _ = search.rerank_exact(ix, rp, refined, q, p2.error_bounds)
+    want_d, want_i = search.topk_pack(d, i, 10)
+    sr = search.Searcher(ix, batch, tp.capacity(top_n), top_n, 1)
+    sr.set_pq2(p2, top_l)
+    got_i, got_d = sr.run_host(q.cpu().numpy(), tp, rp, np.array([s.medoid], np.uint32))[:2]
+    sr.close()
+    assert np.array_equal(got_i, np_u32(want_i))
+    assert np.array_equal(got_d.view(np.uint32), np_u32(want_d))

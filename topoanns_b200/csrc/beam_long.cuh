@@ -67,7 +67,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
         my_j[r] = r * kBeamThreads + tid - my_k[r] * deg;
     }
     // Marked queries are few: the block looks at the marks of 128 of its queries at a time (one dependent load per query
-    // took 32 us for 10 k queries, the launch now takes 13).
+    // took 32 us for 10 k queries).
     const uint32_t group = a.only_marked != 0u ? (uint32_t)kBeamThreads : 1u;
     for (uint64_t first = blockIdx.x; first < a.num_queries; first += (uint64_t)gridDim.x * group) {
     if (a.only_marked != 0u) {
@@ -77,9 +77,9 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
         if (lane == 0) s_marks[warp] = marks;
         __syncthreads();
     }
-    for (uint32_t g = 0; g < group; ++g) {
-    if (a.only_marked != 0u && ((s_marks[g >> 5] >> (g & 31u)) & 1u) == 0u) continue;
-    const uint64_t q = first + (uint64_t)g * gridDim.x;
+    for (uint32_t w = 0; w < group; w += 32u) {
+    for (uint32_t marks = a.only_marked != 0u ? s_marks[w >> 5] : 1u; marks != 0u; marks &= marks - 1u) {
+    const uint64_t q = first + (uint64_t)(w + __ffs(marks) - 1u) * gridDim.x;
     const uint32_t entry_begin = a.entry_offsets[q];
     const uint32_t num_entries = a.entry_offsets[q + 1] - entry_begin;
 
@@ -452,6 +452,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
             st[0] = visited; st[1] = expanded; st[2] = 0; st[3] = iterations;
             st[4] = valid; st[5] = first_full; st[6] = 0; st[7] = 0;
         }
+    }
     }
     }
     }

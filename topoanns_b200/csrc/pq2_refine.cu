@@ -104,6 +104,132 @@ pq2_refine_kernel(const Cand* __restrict__ cand, const uint32_t* __restrict__ st
     }
 }
 
+// The table-free form for larger batches: one block of 32 warps per SM keeps the second-level pivots in shared memory and
+// eight groups of four warps take a query each. What bounds the form above are the gathers: each lane reads its chunk's pivots
+// (dim / M values) and a cross term from lines of their own, and the L1 cache looks up one line per cycle; with the pivots in
+// shared memory only the cross terms (12.6 MB at M = 48: L2) are left. Four ranks at a time keep four dependent chains
+// (record, code rows, terms) of a warp in flight. The sums are those of the form above, operation for operation.
+constexpr int kPq2Groups = 8, kPq2GroupThreads = 128, kPq2Ranks = 4;
+
+template <int kChunks>   // chunks per lane: ceil(M / 32)
+__global__ void __launch_bounds__(kPq2Groups * kPq2GroupThreads, 1)
+pq2_refine_shared_kernel(const Cand* __restrict__ cand, const uint32_t* __restrict__ stats, uint64_t Q, uint32_t capacity,
+                         uint32_t Lr, uint32_t padded, int has_base, TannShards base_codes, TannShards pq2_codes, uint32_t M,
+                         const float* __restrict__ cross, Cand* __restrict__ out, const float* __restrict__ t2_col_major,
+                         const float* __restrict__ mu2, const uint32_t* __restrict__ chunk_offsets,
+                         const float* __restrict__ queries_f32, uint32_t dim) {
+    extern __shared__ __align__(16) float pq2_shared[];
+    const uint32_t lane = threadIdx.x & 31, group = threadIdx.x / kPq2GroupThreads, tid = threadIdx.x % kPq2GroupThreads;
+    const uint32_t warp = tid >> 5;
+    float* pivots = pq2_shared;
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(pivots + (size_t)dim * kCentroids) + (size_t)group * padded;
+    float* sq = reinterpret_cast<float*>(reinterpret_cast<unsigned long long*>(pivots + (size_t)dim * kCentroids) + (size_t)kPq2Groups * padded) + group * dim;
+    constexpr unsigned long long kInvalidKey = 0xff800000ffffffffull;
+    for (uint32_t i = threadIdx.x; i < dim * (kCentroids / 4); i += kPq2Groups * kPq2GroupThreads)
+        reinterpret_cast<float4*>(pivots)[i] = __ldg(reinterpret_cast<const float4*>(t2_col_major) + i);
+    uint32_t first[kChunks], end[kChunks];
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+        const uint32_t m = i * 32 + lane;
+        first[i] = m < M ? __ldg(chunk_offsets + m) : 0u;
+        end[i] = m < M ? __ldg(chunk_offsets + m + 1) : 0u;
+    }
+    __syncthreads();
+    const auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(group + 1u), "n"(kPq2GroupThreads) : "memory"); };
+    // neighbouring queries go to different blocks, so that a batch of few queries is spread over the SMs
+    for (uint64_t q = (uint64_t)group * gridDim.x + blockIdx.x; q < Q; q += (uint64_t)gridDim.x * kPq2Groups) {
+        const uint32_t valid = min(stats[q * 8 + 4], Lr);
+        for (uint32_t i = tid; i < dim; i += kPq2GroupThreads) sq[i] = queries_f32[q * dim + i] - __ldg(mu2 + i);
+        group_sync();
+        for (uint32_t rank0 = warp * kPq2Ranks; rank0 < padded; rank0 += kPq2GroupThreads / 32 * kPq2Ranks) {
+            uint32_t id[kPq2Ranks];
+            float dist[kPq2Ranks], partial[kPq2Ranks];
+            uint32_t rc[kPq2Ranks][kChunks];
+            float term[kPq2Ranks][kChunks];
+#pragma unroll
+            for (int u = 0; u < kPq2Ranks; ++u) {
+                id[u] = kInvalid;
+                dist[u] = 0.0f;
+                if (rank0 + u < valid) {
+                    const Cand c = cand[q * capacity + rank0 + u];
+                    id[u] = RawId(c.id);
+                    dist[u] = c.dist;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kPq2Ranks; ++u) {
+#pragma unroll
+                for (int i = 0; i < kChunks; ++i) {
+                    const uint32_t m = i * 32 + lane;
+                    rc[u][i] = 0;
+                    uint32_t bc = 0;
+                    if (id[u] != kInvalid && m < M) {
+                        rc[u][i] = __ldg(ShardRow(pq2_codes, id[u], M) + m);
+                        if (has_base) bc = __ldg(ShardRow(base_codes, id[u], M) + m);
+                    }
+                    rc[u][i] |= bc << 8;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kPq2Ranks; ++u) {
+#pragma unroll
+                for (int i = 0; i < kChunks; ++i) {
+                    const uint32_t m = i * 32 + lane;
+                    term[u][i] = 0.0f;
+                    if (has_base && id[u] != kInvalid && m < M)
+                        term[u][i] = __ldg(cross + ((size_t)m * kCentroids + (rc[u][i] >> 8)) * kCentroids + (rc[u][i] & 255u));
+                    rc[u][i] &= 255u;
+                }
+                partial[u] = 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < kChunks; ++i) {
+                float entry[kPq2Ranks];
+#pragma unroll
+                for (int u = 0; u < kPq2Ranks; ++u) entry[u] = 0.0f;
+                for (uint32_t k = first[i]; k < end[i]; ++k) {
+                    const float s = sq[k];
+#pragma unroll
+                    for (int u = 0; u < kPq2Ranks; ++u) {
+                        const float diff = pivots[k * kCentroids + rc[u][i]] - s;
+                        entry[u] = fmaf(diff, diff, entry[u]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kPq2Ranks; ++u)
+                    if (i * 32 + lane < M) partial[u] += has_base ? entry[u] + term[u][i] : entry[u];
+            }
+#pragma unroll
+            for (int u = 0; u < kPq2Ranks; ++u) {
+                const float sum = WarpTreeSum(partial[u]);
+                const float d = has_base ? dist[u] + sum : sum;
+                if (lane == 0 && rank0 + u < padded) keys[rank0 + u] = id[u] != kInvalid ? KeyOf(d, id[u]) : kInvalidKey;
+            }
+        }
+        group_sync();
+        for (uint32_t k = 2; k <= padded; k <<= 1) {
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                for (uint32_t t = tid; t < padded / 2; t += kPq2GroupThreads) {
+                    const uint32_t lo = ((t & ~(j - 1)) << 1) | (t & (j - 1));
+                    const uint32_t hi = lo | j;
+                    const bool asc = (lo & k) == 0;
+                    const unsigned long long a = keys[lo], b = keys[hi];
+                    if ((a > b) == asc) { keys[lo] = b; keys[hi] = a; }
+                }
+                group_sync();
+            }
+        }
+        for (uint32_t i = tid; i < Lr; i += kPq2GroupThreads) {
+            const unsigned long long k = keys[i];
+            Cand c;
+            c.dist = FromOrderedBits((uint32_t)(k >> 32));
+            c.id = (uint32_t)k;
+            out[q * Lr + i] = c;
+        }
+        group_sync();
+    }
+}
+
 // X[m][b][r] = 2 * sum_dim (T1[b][dim] + mu1[dim]) * (T2[r][dim] + mu2[dim]), products and sums
 // rounded separately like the host loop of the reference (src/search/search_resources.cpp:52-91).
 __global__ void __launch_bounds__(256)
@@ -134,6 +260,22 @@ cudaError_t LaunchPq2Refine(const void* cand, const uint32_t* stats, uint64_t Q,
     if (Q == 0 || refine_top_l == 0) return cudaSuccess;
     uint32_t padded = 1;
     while (padded < refine_top_l) padded <<= 1;
+    // The pivots take 98 KB at dim = 96; a batch has to be large enough to pay for loading them into every SM. M = 48, one
+    // block per query -> pivots in shared memory, for lists of 16 / 64 / 256: 148 queries 8.8 -> 11.9, 23.8 -> 26.0,
+    // 101.8 -> 85.9 us; 600 queries 14.5 -> 14.7, 34.9 -> 32.4, 108.5 -> 96.7; 10 k queries 115 -> 92, 340 -> 266,
+    // 1229 -> 900. The line is at four queries per SM.
+    const size_t shared = (size_t)dim * kCentroids * 4 + kPq2Groups * ((size_t)padded * 8 + (size_t)dim * 4);
+    if (lut2 == nullptr && selector_bits == nullptr && M <= 96 && Q >= (uint64_t)SmCount() * 4 && shared <= 227u * 1024u &&
+        (reinterpret_cast<uintptr_t>(t2_col_major) & 15u) == 0) {
+        const auto kernel = M <= 32 ? pq2_refine_shared_kernel<1> : (M <= 64 ? pq2_refine_shared_kernel<2> : pq2_refine_shared_kernel<3>);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (e != cudaSuccess) return e;
+        kernel<<<(unsigned)SmCount(), kPq2Groups * kPq2GroupThreads, shared, stream>>>(
+            static_cast<const Cand*>(cand), stats, Q, capacity, refine_top_l, padded, base_codes != nullptr ? 1 : 0,
+            base_codes != nullptr ? *base_codes : TannShards{}, pq2_codes, M, cross_terms, static_cast<Cand*>(out), t2_col_major, mu2,
+            chunk_offsets, queries_f32, dim);
+        return cudaGetLastError();
+    }
     const size_t smem = (size_t)padded * 8 + (lut2 == nullptr ? (size_t)dim * 4 : 0);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(pq2_refine_kernel,
