@@ -1117,7 +1117,7 @@ def main():
                 "h2d_bytes_per_step": q_host_bytes, "d2h_bytes_per_step": int(Q * 10 * 8),
                 "pipeline": f"{n_lanes} searchers on {n_lanes} streams, batches submitted in turn (copies of one overlap kernels of the others)",
                 "one_batch_at_a_time": total_q / (e2e_serial_ms * 1e-3)},
-        "gpu_launches": 5 * args.steps,  # rvq, beam, float->uint8 check, rerank, top-k pack
+        "gpu_launches": 6 * args.steps,  # rvq, pivot layout, beam, float->uint8 check, rerank, top-k pack (and the repeat of marked queries when the list is longer than top_l)
         "clocks": clocks,
         "roofline": roofline,
     }

@@ -58,6 +58,8 @@ bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan) 
     plan->long_smem = plan->two_lists ? two : one;
     plan->smem = plan->long_smem;
     if (plan->long_smem > 227u * 1024u - 512u) return false;
+    // Long form -> short form on the same index: L = 64 (M = 48) 307 -> 219 us for 500 queries, L = 256 9.74 -> 7.2 ms for 10 k.
+    // Lists of 512 would need 16 register pairs per lane, whose merges bound the step: 2.7 -> 6.5 ms for 2 k queries (M = 32).
     plan->list_regs = 0;
     plan->pool_len = 0;
     plan->may_mark = false;
