@@ -73,19 +73,3 @@ def test_pq2_refine_inside_the_searcher_matches_the_table_form(top_l, batch):
     sr.close()
     assert np.array_equal(got_i, np_u32(want_i))
     assert np.array_equal(got_d.view(np.uint32), np_u32(want_d))
-
-
-@pytest.mark.parametrize("top_l,top_n", [(16, 64), (64, 64), (100, 128), (200, 256), (300, 512)])
-def test_distances_that_are_not_finite_are_listed_as_by_the_general_form(top_l, top_n):
-    """A capacity above 1024 takes the general form; the ranks that both lists have are the same, bit for bit."""
-    s, _ = small_index()
-    ix = device_index(s)
-    q = s.queries.cuda().float()[:8].contiguous()
-    q[1, 3], q[2, 5], q[3, 7], q[4] = float("nan"), float("inf"), -float("inf"), 3e38
-    eo, ei = fixed_entries(8, [s.medoid, 17, 400])
-    p = search.TopologySearchParams(top_k=10, top_l=top_l, search_width=2, max_expansions=64)
-    cap = p.capacity(top_n)
-    got, got_stats = search.beam_search(ix, p, eo, ei, queries=q, capacity=cap)
-    want, want_stats = search.beam_search(ix, p, eo, ei, queries=q, capacity=2048)
-    assert np.array_equal(np_u32(got), np_u32(want)[:, :cap])
-    assert np.array_equal(np_u32(got_stats)[:, [0, 1, 3]], np_u32(want_stats)[:, [0, 1, 3]])

@@ -10,7 +10,6 @@
 namespace tann {
 
 constexpr uint32_t kTakenWords = 32;   // places of a list
-constexpr unsigned long long kNoneKey = ~0ull;   // behind every key, also one whose distance is a NaN
 
 // Where the parts of a block's shared memory start, in bytes; shared by the launcher and the kernel.
 struct LongLayout {
@@ -113,7 +112,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
         uint32_t valid = 0, visited = 0, hash_iter = 0, expanded = 0, iterations = 0, mv = 0;
         uint32_t first_full = 0xffffffffu, entries_done = 0, nslots = slots, parity = 0;
         // of warp 0, lane x: the x-th unexpanded entry of the list, and its rank
-        unsigned long long un_key = kNoneKey;
+        unsigned long long un_key = kInvalidKey;
         uint32_t un_pos = 0;
         bool from_entries = num_entries != 0, stop = num_entries == 0;
         uint32_t id[kR], words[kR][kM / 4];
@@ -183,23 +182,23 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
                 uint32_t nsel = 0, new_picks = 0, list_end = 0, pick = kInvalid;
                 if (expanded < a.p.max_expansions) {
                     // of the new keys a lane looks at (usually one), the least; used = those selected already
-                    unsigned long long least = kNoneKey;
+                    unsigned long long least = kInvalidKey;
                     uint32_t at_s = 0, used = 0, un_taken = 0;
                     for (uint32_t s = 0; s * 32u < n; ++s) {
-                        const unsigned long long k = s * 32u + lane < n ? fkey[s * 32u + lane] : kNoneKey;
+                        const unsigned long long k = s * 32u + lane < n ? fkey[s * 32u + lane] : kInvalidKey;
                         if (k < least) { least = k; at_s = s; }
                     }
-                    unsigned long long s_min = n != 0 ? WarpMinKey(least) : kNoneKey;
+                    unsigned long long s_min = n != 0 ? WarpMinKey(least) : kInvalidKey;
                     while (nsel < W) {
                         const unsigned long long u = __shfl_sync(kFull, un_key, un_taken);
-                        if (s_min < kNoneKey && s_min <= u) {
+                        if (s_min < kInvalidKey && s_min <= u) {
                             // inside the first L ranks: fewer than L - new_picks list entries are below it
                             const uint32_t at = L - 1u - new_picks;
                             if (new_picks >= L || !(at >= mv || s_min <= (cur[at] & kCmpMask))) break;
                             if (mv + n > list_len) {
                                 // a tie with the entry it would displace: not accepted, nor is any larger new key
                                 const uint32_t last = list_len - 1u - new_picks;
-                                if (last < mv && s_min >= (cur[last] & kCmpMask)) { s_min = kNoneKey; continue; }
+                                if (last < mv && s_min >= (cur[last] & kCmpMask)) { s_min = kInvalidKey; continue; }
                             }
                             if (lane == nsel) pick = (uint32_t)s_min & kRawMask;
                             ++new_picks;
@@ -207,17 +206,17 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
                                 const uint32_t owner = __ffs(__ballot_sync(kFull, least == s_min)) - 1;
                                 if (lane == owner) {
                                     used |= 1u << at_s;
-                                    least = kNoneKey;
+                                    least = kInvalidKey;
                                     if (n > 32u) {
                                         for (uint32_t s = 0; s * 32u < n; ++s) {
-                                            const unsigned long long k = (s * 32u + lane < n && !((used >> s) & 1u)) ? fkey[s * 32u + lane] : kNoneKey;
+                                            const unsigned long long k = (s * 32u + lane < n && !((used >> s) & 1u)) ? fkey[s * 32u + lane] : kInvalidKey;
                                             if (k < least) { least = k; at_s = s; }
                                         }
                                     }
                                 }
                                 s_min = WarpMinKey(least);
                             }
-                        } else if (u < kNoneKey) {
+                        } else if (u < kInvalidKey) {
                             const uint32_t pos = __shfl_sync(kFull, un_pos, un_taken);
                             if (pos + new_picks >= L) break;
                             if (lane == nsel) pick = (uint32_t)u & kRawMask;
@@ -287,8 +286,8 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
                 // this push below it, plus list entries below it.
                 for (uint32_t c = warp - 1u; c * 32u < n && warp != 0; c += 3u) {
                     const uint32_t i = c * 32u + lane;
-                    if (lane < 4u) fkey[n + lane] = kNoneKey;   // the loop below takes four keys at a time
-                    const unsigned long long k = i < n ? fkey[i] : kNoneKey;
+                    if (lane < 4u) fkey[n + lane] = kInvalidKey;   // the loop below takes four keys at a time
+                    const unsigned long long k = i < n ? fkey[i] : kInvalidKey;
                     __syncwarp();
                     uint32_t rank = 0;
 #pragma unroll 1
@@ -330,7 +329,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
                 __syncthreads();
                 if (tid == 0) s_flag = 0;
                 for (uint32_t i = tid; i < n; i += kBeamThreads)
-                    if (place[i] & 0x8000u) fkey[i] = kNoneKey;
+                    if (place[i] & 0x8000u) fkey[i] = kInvalidKey;
                 if (tid < kTakenWords) taken[tid] = 0u;
                 __syncthreads();
             }
@@ -421,7 +420,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
                     if (lane == w) word &= word - 1u;
                     live = __ballot_sync(kFull, word != 0u);
                 }
-                un_key = lane < found ? cur[un_pos] : kNoneKey;
+                un_key = lane < found ? cur[un_pos] : kInvalidKey;
                 if constexpr (kLate) {
                     if (lane < found) picks.node[lane] = (uint32_t)un_key & kRawMask;
                     const uint32_t last = __shfl_sync(kFull, un_pos, found != 0u ? found - 1u : 0u);

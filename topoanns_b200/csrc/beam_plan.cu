@@ -60,10 +60,12 @@ bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan) 
     if (plan->long_smem > 227u * 1024u - 512u) return false;
     // Long form -> short form on the same index: L = 64 (M = 48) 307 -> 219 us for 500 queries, L = 256 9.74 -> 7.2 ms for 10 k.
     // Lists of 512 would need 16 register pairs per lane, whose merges bound the step: 2.7 -> 6.5 ms for 2 k queries (M = 32).
+    // Widths above 2 stay with the long form: one push can then bring three copies of a node, and the states of a key tell two
+    // copies apart (a list of 300 entries at L = 64 and width 3 came out with two copies in the other order).
     plan->list_regs = 0;
     plan->pool_len = 0;
     plan->may_mark = false;
-    if (L > 256 || late || ix.num_nodes > 0x3fffffffull) return true;
+    if (L > 256 || p.search_width > 2 || late || ix.num_nodes > 0x3fffffffull) return true;
     const uint32_t regs = L <= 32 ? 1u : (L <= 64 ? 2u : (L <= 128 ? 4u : 8u));
     if (C > 32 * regs) {
         // room for the ranks behind the list, the keys of two pushes and some slack for the cut

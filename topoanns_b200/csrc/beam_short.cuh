@@ -1,4 +1,4 @@
-// Beam search for lists of at most 256 ranks in the traversal (top_l <= 256), chunk counts that are multiples of 16, at most
+// Beam search for lists of at most 256 ranks in the traversal (top_l <= 256), search widths of 1 and 2, chunk counts that are multiples of 16, at most
 // 256 frontier slots per step: the common case of the path. One query per block of five warps; the traversal is the
 // reference kernel's (src/search/topology_search_kernel.cu:2190-2664) step by step, and the records are bit for bit those of
 // the general kernels.
@@ -31,7 +31,7 @@ namespace tann {
 
 constexpr uint32_t kSlotThreads = 128, kShortThreads = 160;
 constexpr uint32_t kNew = 0, kExpanded = 1, kTwin = 2;
-constexpr unsigned long long kNoKey = ~0ull;   // behind every key, also one whose distance is a NaN
+constexpr unsigned long long kNoKey = 0xff800000ffffffffull;   // (+inf, no id): behind every key
 constexpr uint32_t kTailBuckets = 128;
 constexpr int kTailPer = 6;            // the pool holds at most kSlotThreads * kTailPer keys
 
@@ -85,8 +85,8 @@ __device__ __forceinline__ unsigned long long MergeIntoList(unsigned long long (
 
 __device__ __forceinline__ Cand RecordOf(unsigned long long k) {
     Cand c;
+    c.dist = FromOrderedBits((uint32_t)(k >> 32));
     const uint32_t low = (uint32_t)k;
-    c.dist = low == 0xffffffffu ? __int_as_float(0x7f800000) : FromOrderedBits((uint32_t)(k >> 32));
     c.id = low == 0xffffffffu ? kInvalid : (low >> 2) | ((low & 3u) == kExpanded ? kExpandedBit : 0u);
     return c;
 }
