@@ -983,6 +983,8 @@ void orc_rerank_learned(const void* cand_in, uint64_t Q, uint32_t capacity, uint
                     stop_prefix = processed;
                 }
             }
+            // a stage whose k-th distance was not finite is left behind unevaluated: windows always move on
+            while (use_schedule && !stop && stage < ls.num_stages && ls.stage_prefixes[stage] <= processed) ++stage;
             if (use_schedule && !stop)
                 next_prefix = stage < ls.num_stages ? std::min(budget, ls.stage_prefixes[stage])
                                                     : std::min(budget, processed + tile);

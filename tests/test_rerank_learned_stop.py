@@ -139,6 +139,33 @@ def test_checker_rule_on_a_hand_made_case():
     assert r["ids"][0].tolist() == [0, 1] and int(r["stop_prefixes"][0]) == 24
 
 
+def _few_candidates(top_k, top_n=24):
+    """The hand-made case with lists in which the k-th distance stays infinite at one or more stage boundaries: fewer than
+    top_k valid candidates in front, in the middle or in the whole list, and an infinite query."""
+    cand, _, pages, vpp, vb = _hand_case()
+    lists = np.repeat(cand, 6, axis=0)
+    lists[0, top_k - 1:, 1] = INVALID         # never top_k candidates
+    lists[1, :, 1] = INVALID                  # none at all
+    lists[2, :9, 1] = INVALID                 # none before the second stage
+    lists[3, 1:12, 1] = INVALID               # one, then none up to the second stage
+    lists[4, ::2, 1] = INVALID                # every second rank
+    q = np.zeros((6, 1), np.float32)
+    q[5] = np.inf                             # distances that are infinite
+    return lists, q, pages, vpp, vb
+
+
+@pytest.mark.parametrize("top_k", [2, 7])
+def test_checker_moves_on_when_the_kth_distance_is_not_finite(top_k):
+    cand, q, pages, vpp, vb = _few_candidates(top_k)
+    m = _stop([8, 12, 16], 4, {1: -4.0}, 1.0, -100.0, top_k=top_k)
+    r = orc.rerank_learned(cand, q, pages, np.float32, model=m, top_n=24, top_k=top_k, tile=4, vectors_per_page=vpp,
+                           page_bytes=4096, vector_bytes=vb)
+    assert r["stop_prefixes"].tolist() == [24] * 6 and r["stop_flags"].tolist() == [0] * 6
+    evaluated = {2: [0, 0, 2, 1, 3, 0], 7: [0, 0, 1, 0, 1, 0]}[top_k]
+    assert r["checkpoint_counts"].tolist() == evaluated
+    assert r["ids"][2].tolist() == list(range(top_k)) and r["ids"][1].tolist() == [INVALID] * top_k
+
+
 # ---- GPU: kernel against the checker -------------------------------------------------------------
 
 def _gpu_imports():
@@ -186,6 +213,39 @@ def test_hand_made_case_on_the_gpu():
         got = search.rerank_exact_learned_stop(
             ix, rp, dcand, dq, model=_as_capi(m, capi) if m is not None else None,
             replay_stop_prefixes=torch.from_numpy(replay.view(np.int32)).cuda() if replay is not None else None)
+        _compare(got, want, gs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("top_k,top_n", [(2, 24), (7, 24), (33, 80), (7, 600)])
+def test_kernels_move_on_when_the_kth_distance_is_not_finite(top_k, top_n):
+    """Both forms of the kernel (one warp per query up to top_k = 32 and 512 ranks, else one block)."""
+    torch, capi, search, gs = _gpu_imports()
+    n = top_n
+    vectors = (np.arange(n, dtype=np.float32) + 1).reshape(n, 1)
+    pages, vpp, vb = pipeline.vectors_to_pages(vectors)
+    ix = search.device_index_from_arrays(
+        adjacency=np.full((n, 64), INVALID, np.uint32), codes=np.zeros((n, 1), np.uint8), vectors=vectors,
+        pq_tables_row_major=np.zeros((256, 1), np.float32), pq_centroid=np.zeros(1, np.float32),
+        pq_chunk_offsets=np.array([0, 1], np.uint32))
+    cand = np.zeros((6, n, 2), np.uint32)
+    cand[:, :, 0] = np.arange(n, dtype=np.float32).view(np.uint32)
+    cand[:, :, 1] = np.arange(n - 1, -1, -1, dtype=np.uint32)
+    cand[0, top_k - 1:, 1] = INVALID
+    cand[1, :, 1] = INVALID
+    cand[2, :n // 3, 1] = INVALID
+    cand[3, 1:n // 2, 1] = INVALID
+    cand[4, ::2, 1] = INVALID
+    q = np.zeros((6, 1), np.float32)
+    q[5] = np.inf
+    stages = [n // 6, n // 4, n // 3, n // 2, n - 1]
+    rp = search.RerankExactParams(top_k=top_k, top_n=n, rank_tile_size=4)
+    for threshold in (-100.0, -0.5):
+        m = _stop(stages, 2, {1: -4.0}, 1.0, threshold, top_k=top_k, budget=n)
+        want = orc.rerank_learned(cand, q, pages, np.float32, top_n=n, top_k=top_k, tile=4, vectors_per_page=vpp,
+                                  page_bytes=4096, vector_bytes=vb, model=m)
+        got = search.rerank_exact_learned_stop(ix, rp, torch.from_numpy(cand.view(np.int32)).cuda(),
+                                               torch.from_numpy(q).cuda(), model=_as_capi(m, capi))
         _compare(got, want, gs)
 
 

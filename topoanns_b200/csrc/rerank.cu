@@ -573,6 +573,14 @@ __device__ __forceinline__ float RerankStopLogit(const TannRerankLearnedStop& c,
     return fmaf(exact_frac, c.linear_weights[12], logit);
 }
 
+// The first stage that lies behind `processed` ranks. A stage is left unevaluated while the k-th distance is not finite (fewer
+// than k candidates so far, or distances that are infinite or NaN); the next window then has to end at a later stage: the
+// schedule would otherwise ask for a window of no ranks over and over.
+__device__ __forceinline__ uint32_t SkipPassedStages(const TannRerankLearnedStop& ls, uint32_t stage, uint32_t processed) {
+    while (stage < ls.num_stages && ls.stage_prefixes[stage] <= processed) ++stage;
+    return stage;
+}
+
 __global__ void __launch_bounds__(kRerankThreads)
 rerank_learned_kernel(const __grid_constant__ TannIndexView ix, TannRerankParams p,
                       const __grid_constant__ TannRerankLearnedStop ls, uint32_t use_schedule, uint32_t evaluate,
@@ -754,6 +762,8 @@ rerank_learned_kernel(const __grid_constant__ TannIndexView ix, TannRerankParams
                     s_stop = 1;
                     s_stop_prefix = processed;
                 } else if (use_schedule) {
+                    stage = SkipPassedStages(ls, stage, processed);
+                    s_stage = stage;
                     s_next = stage < ls.num_stages ? min(budget, ls.stage_prefixes[stage]) : min(budget, processed + tile);
                 }
             }
@@ -968,6 +978,7 @@ rerank_learned_warp_kernel(const __grid_constant__ TannIndexView ix, TannRerankP
                     stop = 1;
                     stop_prefix = processed;
                 } else if (use_schedule) {
+                    stage = SkipPassedStages(ls, stage, processed);
                     next = stage < ls.num_stages ? min(budget, ls.stage_prefixes[stage]) : min(budget, processed + tile);
                 }
             }
