@@ -1,9 +1,11 @@
 """The forms of the beam search and of the pq2 refine that a call is sent to by its sizes, at the edges of their ranges."""
+import dataclasses
+
 import numpy as np
 import pytest
 
 from oracle import oracle as orc
-from topoanns_b200 import search
+from topoanns_b200 import capi, search
 
 from gpu_support import assert_candidates_equal, device_index, fixed_entries, np_u32, small_index
 
@@ -73,3 +75,62 @@ def test_pq2_refine_inside_the_searcher_matches_the_table_form(top_l, batch):
     sr.close()
     assert np.array_equal(got_i, np_u32(want_i))
     assert np.array_equal(got_d.view(np.uint32), np_u32(want_d))
+
+
+def _general_form(ix):
+    """The same index with the neighbour codes in two node-id-range shards: a layout that the general kernels take alone."""
+    ix = search.inline_neighbor_codes(dataclasses.replace(ix))
+    ix.rows_per_shard = (ix.num_nodes + 1) // 2
+    base = ix.neighbor_codes.data_ptr()
+    ix.neighbor_codes_bases = [base, base + ix.rows_per_shard * ix.degree * ix.num_chunks]
+    return ix
+
+
+def _learned_stop(top_l):
+    ls = capi.LearnedStop()
+    ls.enabled, ls.num_stages, ls.top_k, ls.inv_top_l = 1, 3, 10, 1.0 / top_l
+    for i, p in enumerate((12, 16, 24)):
+        ls.stage_prefixes[i] = p
+    for i in range(12):
+        ls.feature_mask[i], ls.weights[i] = 1, 1e-4 * (i - 5)
+    ls.bias = 1.0
+    return ls
+
+
+# Distances that are NaN are not listed (no comparison with them holds), infinite ones are, by id. Where a list has them, the
+# count of valid entries runs ahead of the list.
+@pytest.mark.parametrize("chunks", [32, 48])
+@pytest.mark.parametrize("top_l,width,top_n,learned", [(300, 2, 64, False), (400, 1, 1024, False), (64, 4, 64, False), (64, 2, 64, True),
+                                                       (100, 2, 512, True), (200, 4, 256, True)])
+def test_distances_that_are_not_finite_in_long_lists(chunks, top_l, width, top_n, learned):
+    _not_finite(chunks, top_l, width, top_n, learned)
+
+
+def _not_finite(chunks, top_l, width, top_n, learned):
+    s, _ = _index(chunks)
+    ix = device_index(s)
+    q = s.queries.cuda().float()[:12].clone()   # (the index is shared by other tests)
+    lut = search.lut_build(ix, q)
+    rng = np.random.default_rng(top_l)
+    lut[1, 3] = float("nan")                    # every distance
+    lut[2, 5, rng.permutation(256)[:128].tolist()] = float("nan")   # half of them
+    lut[3, 7, ::3] = float("inf")
+    lut[4] = 3e38                               # sums that overflow
+    lut[5, 0, ::2], lut[5, 1, ::2] = float("nan"), float("inf")
+    lut[6, :, 200:] = float("nan")
+    lut[7, 9, :250] = float("nan")              # the list stays far shorter than the count of valid entries
+    qn = q.clone()
+    qn[1, 3], qn[2, 5], qn[3, 7], qn[4], qn[5, 0], qn[5, 1] = float("nan"), float("inf"), -float("inf"), 3e38, float("nan"), float("inf")
+    eo, ei = fixed_entries(12, [s.medoid, 17, 400])
+    p = search.TopologySearchParams(top_k=10, top_l=top_l, search_width=width, max_expansions=512,
+                                    learned_stop=_learned_stop(top_l) if learned else None)
+    cap = p.capacity(top_n)
+    for entries in ((eo, ei), fixed_entries(12, [s.medoid]), fixed_entries(12, range(50, 201))):
+        for kw in (dict(lut=lut), dict(queries=qn)):
+            want, want_stats = search.beam_search(_general_form(ix), p, *entries, capacity=cap, **kw)
+            for form in (ix, search.inline_neighbor_codes(dataclasses.replace(ix))):
+                got, got_stats = search.beam_search(form, p, *entries, capacity=cap, **kw)
+                assert_candidates_equal(got, got_stats, np_u32(want), np_u32(want_stats))
+            w = np_u32(want)
+            assert (w[1, :, 1] == 0xFFFFFFFF).all() and np_u32(want_stats)[1, 4] == min(cap, entries[1].numel() // 12)
+            assert not np.isnan(w[:, :, 0].view(np.float32)).any()

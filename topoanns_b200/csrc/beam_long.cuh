@@ -101,6 +101,8 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
             picks.count = 0; picks.new_picks = 0; picks.list_end = 0;
         }
         if constexpr (kLate) {
+            // the learned stop reads ranks up to `valid`, which are invalid from `mv` on
+            for (uint32_t i = tid; i < list_len; i += kBeamThreads) cur[i] = nxt[i] = kInvalidKey;
             if (tid == 0) {
                 ctl.ls_stage = 0; ctl.ls_has_prev = 0; ctl.ls_topk_changed = 0;
                 ctl.ls_prev_dk = __int_as_float(0x7f800000);
@@ -155,7 +157,9 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
                 key[r] = ((unsigned long long)OrderedBits(AdcXor<kM>(smem_raw, words[r], offs)) << 32) | id[r];
             }
             // ---- which new keys can enter the list -------------------------------------------------------------------------
-            const unsigned long long thr = mv == list_len ? (cur[list_len - 1] & kCmpMask) : ~0ull;
+            // A NaN distance (its key is behind the invalid one) never enters, as in the general form: its slot counts as visited
+            // and as valid, so that `valid` may run ahead of `mv`.
+            const unsigned long long thr = mv == list_len ? (cur[list_len - 1] & kCmpMask) : kInvalidKey;
             uint32_t ballots[kR], mine = 0;
 #pragma unroll
             for (int r = 0; r < kR; ++r) {
