@@ -3,6 +3,7 @@ import dataclasses
 
 import numpy as np
 import pytest
+import torch
 
 from oracle import oracle as orc
 from topoanns_b200 import capi, search
@@ -44,6 +45,40 @@ def test_beam_search_at_the_edges_of_the_list_widths(chunks, top_l, width, top_n
         if layout == "neighbor_codes":
             ix = search.inline_neighbor_codes(ix)
         cand, stats = search.beam_search(ix, p, eo, ei, queries=q, capacity=cap)
+        assert_candidates_equal(cand, stats, want, want_stats)
+
+
+def _shared_neighbours(chunks, degree, nodes=3000, window=160, seed=5):
+    """A graph in which parents share many neighbours, so that one push brings copies of a node and later ones bring it again; the
+    codes are random, so that the copies end up anywhere in the list."""
+    rng = np.random.default_rng(seed)
+    adjacency = np.stack([(i + rng.permutation(window)[:degree] - window // 2) % nodes for i in range(nodes)]).astype(np.uint32)
+    adjacency[:, :4] = rng.integers(0, nodes, (nodes, 4))
+    codes = rng.integers(0, 256, (nodes, chunks)).astype(np.uint8)
+    ix = search.device_index_from_arrays(
+        adjacency=adjacency, codes=codes, vectors=np.zeros((nodes, chunks), np.float32),
+        pq_tables_row_major=rng.normal(size=(256, chunks)).astype(np.float32), pq_centroid=np.zeros(chunks, np.float32),
+        pq_chunk_offsets=np.arange(chunks + 1, dtype=np.uint32))
+    return ix, adjacency, codes, rng
+
+
+# lists that end at top_l and lists that go on behind it, where copies of one node in different states (expanded or not) meet the
+# end of the list; steps of up to 128 and of up to 256 slots, entries that repeat
+@pytest.mark.parametrize("chunks,degree,window,batch", [(32, 32, 80, 3000), (48, 64, 160, 400), (96, 32, 80, 400), (32, 128, 200, 400),
+                                                        (48, 96, 160, 300), (96, 128, 200, 300)])
+@pytest.mark.parametrize("top_l,width,capacity", [(5, 2, 8), (5, 1, 32), (16, 2, 32), (32, 2, 32), (32, 1, 128), (32, 2, 128), (33, 2, 64),
+                                                  (64, 2, 64), (64, 2, 256), (100, 2, 128), (128, 2, 256), (128, 2, 512), (200, 1, 256),
+                                                  (256, 2, 256)])
+def test_copies_of_a_node_across_the_end_of_the_list(chunks, degree, window, batch, top_l, width, capacity):
+    ix, adjacency, codes, rng = _shared_neighbours(chunks, degree, window=window)
+    q = torch.from_numpy(rng.normal(size=(batch, chunks)).astype(np.float32)).cuda()
+    eo, ei = fixed_entries(batch, [3, 700, 700, 1500, 3])
+    lut = search.lut_build(ix, q)
+    want, want_stats = orc.beam_search(adjacency, codes, lut.cpu().numpy(), np_u32(eo), np_u32(ei), top_l=top_l, search_width=width,
+                                       max_expansions=1024, capacity=capacity)
+    p = search.TopologySearchParams(top_k=1, top_l=top_l, search_width=width, max_expansions=1024)
+    for form in (ix, search.inline_neighbor_codes(dataclasses.replace(ix))):
+        cand, stats = search.beam_search(form, p, eo, ei, lut=lut, capacity=capacity)
         assert_candidates_equal(cand, stats, want, want_stats)
 
 
@@ -104,6 +139,12 @@ def _learned_stop(top_l):
                                                        (100, 2, 512, True), (200, 4, 256, True)])
 def test_distances_that_are_not_finite_in_long_lists(chunks, top_l, width, top_n, learned):
     _not_finite(chunks, top_l, width, top_n, learned)
+
+
+@pytest.mark.parametrize("chunks", [32, 48])
+@pytest.mark.parametrize("top_l,width,top_n", [(32, 2, 16), (16, 2, 256), (64, 1, 64), (100, 2, 128), (100, 2, 512), (256, 2, 256)])
+def test_distances_that_are_not_finite_in_short_lists(chunks, top_l, width, top_n):
+    _not_finite(chunks, top_l, width, top_n, False)
 
 
 def _not_finite(chunks, top_l, width, top_n, learned):

@@ -20,8 +20,6 @@ struct BeamArgs {
     uint32_t* status;
     // of beam_short_kernel and beam_long_kernel:
     uint32_t list_len, two_lists;   // long: entries of the list, whether it is double-buffered
-    uint32_t pool_len;              // short: entries of the tail's pool (0 = none)
-    uint32_t only_marked;           // long: search only the queries that beam_short_kernel marked in their statistics
     const float* pivots_packed;  // PackPivots() of the index's pivots, or nullptr
 };
 

@@ -37,7 +37,7 @@ struct LongPicks {
 // kKind: 0 = codes gathered by id, 1 = neighbour-code layout, 2 = codes and adjacency in node-id-range shards.
 // kR: slots per thread (ceil(W * degree / 128)). kLate: the learned stop looks at the merged list before nodes are selected.
 template <int kM, int kR, int kKind, bool kLate>
-__global__ void __launch_bounds__(kBeamThreads, kM <= 32 ? 5 : (kM <= 48 ? 4 : (kM <= 64 ? 3 : 2)))
+__global__ void __launch_bounds__(kBeamThreads, kM <= 32 ? 5 : (kM <= 48 ? 4 : 2))
 beam_long_kernel(const __grid_constant__ BeamArgs a) {
     constexpr bool kNbr = kKind == 1;
     constexpr bool kOneShard = kKind != 2;
@@ -54,7 +54,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
     uint32_t* taken = reinterpret_cast<uint32_t*>(smem_raw + lay.words);
     uint32_t* unexp = taken + kTakenWords;
     __shared__ uint32_t s_count[2];       // new keys | passing slots << 16 of a push, two pushes in turn
-    __shared__ uint32_t s_flag, s_marks[kBeamThreads / 32];
+    __shared__ uint32_t s_flag;
     __shared__ __align__(16) LongPicks picks;
     __shared__ BeamCtl ctl;
     const LaneOffsets offs(lane);
@@ -66,20 +66,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
         my_k[r] = (r * kBeamThreads + tid) / deg;
         my_j[r] = r * kBeamThreads + tid - my_k[r] * deg;
     }
-    // Marked queries are few: the block looks at the marks of 128 of its queries at a time (one dependent load per query
-    // took 32 us for 10 k queries).
-    const uint32_t group = a.only_marked != 0u ? (uint32_t)kBeamThreads : 1u;
-    for (uint64_t first = blockIdx.x; first < a.num_queries; first += (uint64_t)gridDim.x * group) {
-    if (a.only_marked != 0u) {
-        const uint64_t mine = first + (uint64_t)tid * gridDim.x;
-        const uint32_t marks = __ballot_sync(kFull, mine < a.num_queries && a.out_stats[mine * 8 + 6] != 0u);
-        __syncthreads();   // the marks before are worked off
-        if (lane == 0) s_marks[warp] = marks;
-        __syncthreads();
-    }
-    for (uint32_t w = 0; w < group; w += 32u) {
-    for (uint32_t marks = a.only_marked != 0u ? s_marks[w >> 5] : 1u; marks != 0u; marks &= marks - 1u) {
-    const uint64_t q = first + (uint64_t)(w + __ffs(marks) - 1u) * gridDim.x;
+    for (uint64_t q = blockIdx.x; q < a.num_queries; q += gridDim.x) {
     const uint32_t entry_begin = a.entry_offsets[q];
     const uint32_t num_entries = a.entry_offsets[q + 1] - entry_begin;
 
@@ -456,8 +443,6 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
             st[0] = visited; st[1] = expanded; st[2] = 0; st[3] = iterations;
             st[4] = valid; st[5] = first_full; st[6] = 0; st[7] = 0;
         }
-    }
-    }
     }
     }
 }

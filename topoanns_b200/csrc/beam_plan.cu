@@ -40,6 +40,7 @@ cudaError_t LaunchPackPivots(const float* col_major, uint32_t M, uint32_t dim, f
 static uint32_t ResidentBlocks(uint32_t smem) { return (228u * 1024u) / (smem + 1024u + 512u); }
 
 bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan) {
+    *plan = FastPlan{};
     const uint32_t M = ix.num_chunks, C = p.candidate_capacity, L = p.top_l;
     const uint32_t slots = p.search_width * ix.degree;
     const bool late = p.learned_stop.enabled != 0;
@@ -51,34 +52,20 @@ bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan) 
     plan->kind = sharded ? 2 : (nbr ? 1 : 0);
     plan->rounds = slots > 128u ? 2u : 1u;
     plan->late = late;
-    // the long form also repeats the queries the short form gives up on
+    // Long form -> short form on the same index: L = 64 (M = 48) 307 -> 219 us for 500 queries, L = 256 9.74 -> 7.2 ms for 10 k.
+    // Lists of 512 would need 16 register pairs per lane, whose merges bound the step: 2.7 -> 6.5 ms for 2 k queries (M = 32).
+    const bool single = p.search_width <= 2 && !late && ix.num_nodes <= 0x3fffffffull;
+    if (single && C >= 32 && C <= 256) {
+        plan->list_regs = C / 32;
+        plan->smem = ShortLayout(M, plan->rounds).total;
+        return plan->smem <= 227u * 1024u - 512u;
+    }
+    if (single && L <= 256 && plan->rounds == 1) return false;
     plan->list_len = C;
     const uint32_t one = LongLayout(M, plan->rounds, C, false).total, two = LongLayout(M, plan->rounds, C, true).total;
     plan->two_lists = ResidentBlocks(two) == ResidentBlocks(one);
-    plan->long_smem = plan->two_lists ? two : one;
-    plan->smem = plan->long_smem;
-    if (plan->long_smem > 227u * 1024u - 512u) return false;
-    // Long form -> short form on the same index: L = 64 (M = 48) 307 -> 219 us for 500 queries, L = 256 9.74 -> 7.2 ms for 10 k.
-    // Lists of 512 would need 16 register pairs per lane, whose merges bound the step: 2.7 -> 6.5 ms for 2 k queries (M = 32).
-    // Widths above 2 stay with the long form: one push can then bring three copies of a node, and the states of a key tell two
-    // copies apart (a list of 300 entries at L = 64 and width 3 came out with two copies in the other order).
-    plan->list_regs = 0;
-    plan->pool_len = 0;
-    plan->may_mark = false;
-    if (L > 256 || p.search_width > 2 || late || ix.num_nodes > 0x3fffffffull) return true;
-    const uint32_t regs = L <= 32 ? 1u : (L <= 64 ? 2u : (L <= 128 ? 4u : 8u));
-    if (C > 32 * regs) {
-        // room for the ranks behind the list, the keys of two pushes and some slack for the cut
-        const uint32_t want = C - 32 * regs + 64 + 256 * plan->rounds, most = kSlotThreads * kTailPer;
-        plan->pool_len = want < most ? want : most;
-        if (plan->pool_len < C - 32 * regs + 64 + 128 * plan->rounds) { plan->pool_len = 0; return true; }
-    }
-    const uint32_t smem = ShortLayout(M, plan->rounds, plan->pool_len).total;
-    if (smem > 227u * 1024u - 512u) { plan->pool_len = 0; return true; }
-    plan->list_regs = regs;
-    plan->may_mark = C > L;
-    plan->smem = smem;
-    return true;
+    plan->smem = plan->two_lists ? two : one;
+    return plan->smem <= 227u * 1024u - 512u;
 }
 
 static cudaError_t LaunchBeamKernel(BeamKernelFn k, const BeamArgs& a, uint32_t grid, uint32_t threads, uint32_t smem, cudaStream_t stream) {
@@ -92,23 +79,16 @@ cudaError_t LaunchFast(BeamArgs a, const FastPlan& plan, uint64_t num_queries, c
     const uint32_t M = a.ix.num_chunks;
     a.list_len = plan.list_len;
     a.two_lists = plan.two_lists ? 1u : 0u;
-    a.pool_len = plan.pool_len;
-    a.only_marked = 0;
-    uint32_t long_grid = (uint32_t)num_queries;
     if (plan.list_regs != 0) {
         BeamKernelFn k = M == 32   ? PickShort32(plan.rounds, plan.kind, plan.list_regs)
                          : M == 48 ? PickShort48(plan.rounds, plan.kind, plan.list_regs)
                                    : PickShort96(plan.rounds, plan.kind, plan.list_regs);
-        const cudaError_t e = LaunchBeamKernel(k, a, (uint32_t)num_queries, kShortThreads, plan.smem, stream);
-        if (e != cudaSuccess || !plan.may_mark) return e;
-        a.only_marked = 1;
-        const uint32_t most = (uint32_t)SmCount();
-        long_grid = long_grid < most ? long_grid : most;
+        return LaunchBeamKernel(k, a, (uint32_t)num_queries, kShortThreads, plan.smem, stream);
     }
     BeamKernelFn k = M == 32   ? PickLong32(plan.rounds, plan.kind, plan.late)
                      : M == 48 ? PickLong48(plan.rounds, plan.kind, plan.late)
                                : PickLong96(plan.rounds, plan.kind, plan.late);
-    return LaunchBeamKernel(k, a, long_grid, kBeamThreads, plan.long_smem, stream);
+    return LaunchBeamKernel(k, a, (uint32_t)num_queries, kBeamThreads, plan.smem, stream);
 }
 
 uint32_t FastBlocksPerSm(const FastPlan& plan) { return ResidentBlocks(plan.smem); }

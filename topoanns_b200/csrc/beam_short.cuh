@@ -1,5 +1,5 @@
-// Beam search for lists of at most 256 ranks in the traversal (top_l <= 256), search widths of 1 and 2, chunk counts that are multiples of 16, at most
-// 256 frontier slots per step: the common case of the path. One query per block of five warps; the traversal is the
+// Beam search for lists of 32, 64, 128 or 256 entries (the candidate capacity), search widths of 1 and 2, 32, 48 or 96 chunks, at
+// most 256 frontier slots per step: the common case of the path. One query per block of five warps; the traversal is the
 // reference kernel's (src/search/topology_search_kernel.cu:2190-2664) step by step, and the records are bit for bit those of
 // the general kernels.
 //
@@ -13,16 +13,13 @@
 //   push's new keys below the list's last one. The list warp picks them right behind the one barrier after the table sums;
 //   the slot warps issue the next loads and the list warp merges the new keys meanwhile: a sort of 32 keys across the
 //   lanes, one split against the end of the list and a bitonic merge.
-// * Lazy tail. Ranks from 32 * kList on never influence the traversal. When the caller wants a longer list they are kept in
-//   an unsorted pool, cut when it is full and sorted at the end.
 //
 // Keys: distance bits (order-preserving) << 32 | id << 2 | state, so that one 64-bit comparison orders copies of one node
-// (they have the same distance) as an eagerly merged list holds them: newest first. Copies within the first top_l ranks come
-// from one push only (anything else there is in the visited filter); when the last selected node has a twin that was not
-// selected, the twin becomes kTwin and stays behind it. Copies behind rank top_l are revisits: they are new (kNew) and lie in
-// front of the older, expanded ones. What the keys cannot tell is which copies an eagerly cut list drops when copies with
-// different states lie across its end; such a query (about one in 10^5) is marked in its statistics and searched again by
-// the general kernel.
+// (they have the same distance) as a merged list holds them: newest first. Copies within the first top_l ranks come from one
+// push only (anything else there is in the visited filter); when the last selected node has copies that were not selected,
+// these become kTwin and stay behind it. Copies behind rank top_l are revisits: they are new (kNew) and lie in front of the
+// older ones, expanded or not. Whether a new key enters a full list is decided without the states: a tie with the entry that it
+// would displace keeps the old one (:1338-1424).
 #pragma once
 
 #include "beam_table.cuh"
@@ -30,35 +27,19 @@
 namespace tann {
 
 constexpr uint32_t kSlotThreads = 128, kShortThreads = 160;
-constexpr uint32_t kNew = 0, kExpanded = 1, kTwin = 2;
-constexpr unsigned long long kNoKey = 0xff800000ffffffffull;   // (+inf, no id): behind every key
-constexpr uint32_t kTailBuckets = 128;
-constexpr int kTailPer = 6;            // the pool holds at most kSlotThreads * kTailPer keys
+constexpr uint32_t kNew = 0, kExpanded = 1, kTwin = 2, kLate = 3;
+constexpr unsigned long long kNoKey = 0xff800000ffffffffull;   // (+inf, no id): behind every key that enters a list
 
 __device__ __forceinline__ void SlotSync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ void BlockSync() { asm volatile("bar.sync 0, 160;" ::: "memory"); }
 
-// Sorts one key per lane, descending.
-__device__ __forceinline__ unsigned long long WarpSortDescending(unsigned long long k, uint32_t lane) {
-#pragma unroll
-    for (uint32_t size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            const unsigned long long o = __shfl_xor_sync(kFull, k, stride);
-            const bool keep_max = ((lane & stride) == 0) == ((lane & size) == 0 || size == 32);
-            if ((o > k) == keep_max) k = o;
-        }
-    }
-    return k;
-}
-
-// Merges 32 keys (one per lane, descending) into the ascending list; returns the 32 largest of both (in no order).
+// Merges 32 keys (one per lane, descending) into the ascending list, which keeps the smallest of both.
 template <int kList>
-__device__ __forceinline__ unsigned long long MergeIntoList(unsigned long long (&list)[kList], unsigned long long k, uint32_t lane) {
-    // list's last 32 ascending against the new keys descending: the smaller halves, with the rest, form a bitonic sequence
-    const bool less = k < list[kList - 1];
-    const unsigned long long out = less ? list[kList - 1] : k;
-    if (less) list[kList - 1] = k;
+__device__ __forceinline__ void MergeIntoList(unsigned long long (&list)[kList], unsigned long long k, uint32_t lane, unsigned long long mask) {
+    // The list's last 32 ascending against the new keys descending: the smaller halves, with the rest, form a bitonic sequence.
+    // This is also the test of an eager merge, new key number x against the entry x places in front of the last, and with the
+    // states masked out a tie keeps the old entry, as there.
+    if (k < (list[kList - 1] & mask)) list[kList - 1] = k;
 #pragma unroll
     for (int stride = kList / 2; stride > 0; stride >>= 1) {
 #pragma unroll
@@ -80,7 +61,6 @@ __device__ __forceinline__ unsigned long long MergeIntoList(unsigned long long (
             if ((o > list[r]) == keep_max) list[r] = o;
         }
     }
-    return out;
 }
 
 __device__ __forceinline__ Cand RecordOf(unsigned long long k) {
@@ -91,216 +71,67 @@ __device__ __forceinline__ Cand RecordOf(unsigned long long k) {
     return c;
 }
 
-// ---- the tail --------------------------------------------------------------------------------------------------------------
-struct TailScratch {
-    uint32_t* hist;     // [kTailBuckets + 1]
-    uint32_t* range;    // [2]
-    uint32_t* counts;   // [32]
-};
-
-__device__ __forceinline__ uint32_t TailBucket(unsigned long long k, uint32_t lo, uint32_t inv) {
-    const uint32_t off = (uint32_t)(k >> 32) - lo;
-    return min(inv == 0u ? off : __umulhi(off, inv), kTailBuckets - 1u);
+// Sorts a list that is sorted except for the states of copies: neighbours are exchanged until none is out of order.
+template <int kList>
+__device__ __forceinline__ void SortCopies(unsigned long long (&list)[kList], uint32_t lane) {
+    bool any;
+    do {
+        bool mine = false;
+#pragma unroll
+        for (int r = 0; r < kList; ++r) {   // ranks 2 i and 2 i + 1
+            const unsigned long long o = __shfl_xor_sync(kFull, list[r], 1);
+            if ((lane & 1u) ? o > list[r] : o < list[r]) { list[r] = o; mine = true; }
+        }
+        unsigned long long before[kList], behind[kList];
+#pragma unroll
+        for (int r = 0; r < kList; ++r) {
+            before[r] = __shfl_sync(kFull, list[r], (lane + 31u) & 31u);
+            behind[r] = __shfl_sync(kFull, list[r], (lane + 1u) & 31u);
+        }
+#pragma unroll
+        for (int r = 0; r < kList; ++r) {   // ranks 2 i + 1 and 2 i + 2
+            const unsigned long long b = lane == 0u ? (r == 0 ? 0ull : before[r - (r > 0)]) : before[r];
+            const unsigned long long f = lane == 31u ? (r == kList - 1 ? ~0ull : behind[r + (r < kList - 1)]) : behind[r];
+            if ((lane & 1u) ? f < list[r] : b > list[r]) { list[r] = (lane & 1u) ? f : b; mine = true; }
+        }
+        any = __any_sync(kFull, mine);
+    } while (any);
 }
-
-// Cuts the n keys of the pool to the smallest `room` (a few more where keys fall into one bucket: only whole buckets of the
-// distance are dropped, so every copy of a kept key is kept) and, at the end of the search (`sort`), sorts them.
-// Returns the number of keys kept; *bound gets the largest distance bits kept. The slot warps call.
-static __device__ __noinline__ uint32_t CutTail(unsigned long long* pool, const TailScratch s, uint32_t n, uint32_t room, bool sort,
-                                         uint32_t* bound) {
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    static_assert(kTailBuckets == kSlotThreads, "one bucket counter per thread");
-    uint32_t lo = 0xffffffffu, hi = 0;
-    if (tid < 2) s.range[tid] = tid == 0 ? 0xffffffffu : 0u;
-    SlotSync();
-#pragma unroll 1
-    for (uint32_t i = tid; i < n; i += kSlotThreads) {
-        const uint32_t b = (uint32_t)(pool[i] >> 32);
-        lo = min(lo, b);
-        hi = max(hi, b);
-    }
-    lo = __reduce_min_sync(kFull, lo);
-    hi = __reduce_max_sync(kFull, hi);
-    if (lane == 0) { atomicMin(&s.range[0], lo); atomicMax(&s.range[1], hi); }
-    SlotSync();
-    lo = s.range[0];
-    hi = s.range[1];
-    uint32_t inv = 0, kept = n;
-    // Distances are spread unevenly (the first entries lie far out), so the range is narrowed to the buckets that are kept
-    // until these hold little more than `room` keys.
-#pragma unroll 1
-    for (int pass = 0; pass < 4; ++pass) {
-        const uint32_t range = hi - lo;
-        // bucket = (bits - lo) * kTailBuckets / (range + 1), rounded down: monotone in the distance
-        inv = range < kTailBuckets ? 0u : (uint32_t)(((unsigned long long)kTailBuckets << 32) / ((unsigned long long)range + 1));
-        s.hist[tid] = 0;
-        SlotSync();
-#pragma unroll 1
-        for (uint32_t i = tid; i < n; i += kSlotThreads) {
-            const unsigned long long k = pool[i];
-            if ((uint32_t)(k >> 32) <= hi) atomicAdd(&s.hist[TailBucket(k, lo, inv)], 1u);
-        }
-        SlotSync();
-        // every warp: the first bucket with `room` keys up to its end (four buckets per lane)
-        const uint4 c = reinterpret_cast<const uint4*>(s.hist)[lane];
-        const uint32_t sum = c.x + c.y + c.z + c.w;
-        uint32_t incl = sum;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t t = __shfl_up_sync(kFull, incl, off);
-            if (lane >= (uint32_t)off) incl += t;
-        }
-        const uint32_t all = __shfl_sync(kFull, incl, 31);
-        uint32_t last = kTailBuckets - 1u, upto = all;
-        if (all > room) {
-            const uint32_t owner = __ffs(__ballot_sync(kFull, incl >= room)) - 1u;
-            uint32_t run = incl - sum, b = 0;
-            run += c.x;
-            if (run < room) { b = 1; run += c.y; }
-            if (run < room) { b = 2; run += c.z; }
-            if (run < room) { b = 3; run += c.w; }
-            last = __shfl_sync(kFull, lane * 4u + b, owner);
-            upto = __shfl_sync(kFull, run, owner);
-        }
-        kept = upto;
-        if (last == kTailBuckets - 1u) break;
-        // the largest offset of bucket `last`: off * inv < (last + 1) << 32
-        hi = lo + (inv == 0u ? last : (uint32_t)((((unsigned long long)(last + 1u) << 32) - 1u) / inv));
-        if (inv == 0u || kept <= room + 32u) break;
-        SlotSync();   // the counters are read before they are cleared
-    }
-    *bound = hi;
-    SlotSync();
-    // the keys that stay, in the pool's order
-    unsigned long long k[kTailPer];
-    uint32_t stays = 0;
-#pragma unroll
-    for (int u = 0; u < kTailPer; ++u) {
-        const uint32_t i = tid + u * kSlotThreads;
-        bool stay = false;
-        if (u * kSlotThreads < n) {
-            if (i < n) { k[u] = pool[i]; stay = (uint32_t)(k[u] >> 32) <= hi; }
-            const uint32_t b = __ballot_sync(kFull, stay);
-            if (lane == 0) s.counts[u * 4 + warp] = __popc(b);
-        } else if (lane == 0) {
-            s.counts[u * 4 + warp] = 0;
-        }
-        stays |= (stay ? 1u : 0u) << u;
-    }
-    SlotSync();
-    const uint32_t mine = lane < 4u * kTailPer ? s.counts[lane] : 0u;
-#pragma unroll
-    for (int u = 0; u < kTailPer; ++u) {
-        if (u * kSlotThreads < n) {
-            const bool stay = (stays >> u) & 1u;
-            const uint32_t b = __ballot_sync(kFull, stay);
-            const uint32_t before = __reduce_add_sync(kFull, lane < u * 4u + warp ? mine : 0u);
-            if (stay) pool[before + __popc(b & ((1u << lane) - 1u))] = k[u];
-        }
-    }
-    kept = __reduce_add_sync(kFull, mine);
-    s.hist[tid] = 0;
-    SlotSync();
-    if (!sort) return kept;
-    // ---- bucket sort of the kept keys ------------------------------------------------------------------------------------
-    {
-        const uint32_t range = hi - lo;
-        inv = range < kTailBuckets ? 0u : (uint32_t)(((unsigned long long)kTailBuckets << 32) / ((unsigned long long)range + 1));
-    }
-    uint32_t slot[kTailPer];
-#pragma unroll
-    for (int u = 0; u < kTailPer; ++u) {
-        const uint32_t i = tid + u * kSlotThreads;
-        if (i < kept) {
-            k[u] = pool[i];
-            slot[u] = atomicAdd(&s.hist[TailBucket(k[u], lo, inv)], 1u);
-        }
-    }
-    SlotSync();
-    if (warp == 0) {
-        const uint4 c = reinterpret_cast<const uint4*>(s.hist)[lane];
-        const uint32_t sum = c.x + c.y + c.z + c.w;
-        uint32_t incl = sum;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t t = __shfl_up_sync(kFull, incl, off);
-            if (lane >= (uint32_t)off) incl += t;
-        }
-        const uint32_t run = incl - sum;
-        reinterpret_cast<uint4*>(s.hist)[lane] = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
-        if (lane == 31) s.hist[kTailBuckets] = incl;
-    }
-    SlotSync();
-#pragma unroll
-    for (int u = 0; u < kTailPer; ++u) {
-        const uint32_t i = tid + u * kSlotThreads;
-        if (i < kept) {
-            const uint32_t p = s.hist[TailBucket(k[u], lo, inv)] + slot[u];
-            pool[p] = k[u];
-        }
-    }
-    SlotSync();
-#pragma unroll
-    for (int u = 0; u < kTailPer; ++u) {
-        const uint32_t i = tid + u * kSlotThreads;
-        if (i < kept) {
-            const uint32_t bk = TailBucket(k[u], lo, inv);
-            const uint32_t b = s.hist[bk], e = s.hist[bk + 1];
-            const uint32_t own = b + slot[u];   // equal keys in the order they were scattered in
-            uint32_t r = b;
-#pragma unroll 1
-            for (uint32_t j = b; j < e; ++j) r += (pool[j] < k[u] || (pool[j] == k[u] && j < own)) ? 1u : 0u;
-            slot[u] = r;
-        }
-    }
-    SlotSync();
-#pragma unroll
-    for (int u = 0; u < kTailPer; ++u)
-        if (tid + u * kSlotThreads < kept) pool[slot[u]] = k[u];
-    SlotSync();
-    return kept;
-}
-
 
 struct ShortLayout {
-    uint32_t bloom, fkey, pool, total;
-    __host__ __device__ ShortLayout(uint32_t M, uint32_t rounds, uint32_t pool_len) {
+    uint32_t bloom, fkey, total;
+    __host__ __device__ ShortLayout(uint32_t M, uint32_t rounds) {
         bloom = M * kCentroids * 4;
         fkey = bloom + kBloomWords * 4;                      // new keys of a push, two pushes in turn
-        pool = fkey + 2 * kSlotThreads * rounds * 8;
-        total = pool + pool_len * 8;
+        total = fkey + 2 * kSlotThreads * rounds * 8;
     }
 };
 
 // kKind: 0 = codes gathered by id, 1 = neighbour-code layout, 2 = codes and adjacency in node-id-range shards.
 // kR: slots per thread (ceil(W * degree / 128)). kList: list registers per lane of the list warp.
 template <int kM, int kR, int kKind, int kList>
-__global__ void __launch_bounds__(kShortThreads, kM <= 32 ? 5 : (kM <= 48 ? 4 : (kM <= 64 ? 3 : 2)))
+__global__ void __launch_bounds__(kShortThreads, kM <= 32 ? 5 : (kM <= 48 ? 4 : 2))
 beam_short_kernel(const __grid_constant__ BeamArgs a) {
     constexpr bool kNbr = kKind == 1;
     constexpr bool kOneShard = kKind != 2;
     constexpr uint32_t kFresh = kSlotThreads * kR;   // new keys per push at most
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const ShortLayout lay(kM, kR, a.pool_len);
+    const ShortLayout lay(kM, kR);
     uint32_t* bloom = reinterpret_cast<uint32_t*>(smem_raw + lay.bloom);
     unsigned long long* fkey = reinterpret_cast<unsigned long long*>(smem_raw + lay.fkey);
-    unsigned long long* pool = reinterpret_cast<unsigned long long*>(smem_raw + lay.pool);
     __shared__ unsigned long long s_thr;       // last key of the list; a new key behind it cannot enter
     __shared__ __align__(16) uint32_t s_count[4];   // per slot warp: new keys of the push | passing slots << 16
     __shared__ __align__(16) unsigned long long s_sort[32];
-    __shared__ unsigned long long s_open_key[32], s_end[2];   // of the list warp: its first unexpanded keys and their ranks; ranks L - 1, L - 2
-    __shared__ uint32_t s_open_rank[32];
-    __shared__ uint32_t s_pool_n, s_tail_thr, s_fail, s_range[2];
-    __shared__ uint32_t s_nsel, s_cut;         // nodes selected (0 ends the search); the pool is to be cut
-    __shared__ uint32_t s_node[TANN_MAX_SEARCH_WIDTH];
+    __shared__ unsigned long long s_open_key[2], s_end[2];   // of the list warp: its first unexpanded keys and their ranks; ranks L - 1, L - 2
+    __shared__ uint32_t s_open_rank[2];
+    __shared__ uint32_t s_nsel, s_node[2];     // nodes selected (0 ends the search)
     const uint64_t q = blockIdx.x;
     const uint32_t W = a.p.search_width, deg = a.ix.degree, slots = W * deg;
     const uint32_t entry_begin = a.entry_offsets[q];
     const uint32_t num_entries = a.entry_offsets[q + 1] - entry_begin;
     const uint32_t entry_pushes = (num_entries + slots - 1) / slots;
-    const bool tail = a.pool_len != 0;
-    const uint32_t C = a.p.candidate_capacity;
+    constexpr uint32_t C = 32u * kList;        // the candidate capacity
 
     if (warp < 4) {
         // ================================================ slot warps ========================================================
@@ -359,8 +190,8 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 PermuteXor<kM>(lane, words[r]);
                 key[r] = ((unsigned long long)OrderedBits(AdcXor<kM>(smem_raw, words[r], offs)) << 32) | (id[r] << 2);
             }
-            // ---- which new keys go to the list, which into the tail ----------------------------------------------------------
-            uint32_t to_tail[kR], mine = 0, mine_tail = 0;
+            // ---- the new keys that can enter the list ------------------------------------------------------------------------
+            uint32_t mine = 0;
             unsigned long long* segment = fkey + (push & 1u) * kFresh + warp * (32u * kR);
 #pragma unroll
             for (int r = 0; r < kR; ++r) {
@@ -368,23 +199,8 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 const uint32_t b = __ballot_sync(kFull, surv);
                 if (surv) segment[(mine & 0xffffu) + __popc(b & lt)] = key[r];
                 mine += __popc(b) + (__popc(__ballot_sync(kFull, pass[r])) << 16);
-                to_tail[r] = 0;
-                if (tail) {
-                    to_tail[r] = __ballot_sync(kFull, pass[r] && !surv && (uint32_t)(key[r] >> 32) <= s_tail_thr);
-                    mine_tail += __popc(to_tail[r]);
-                }
             }
             if (lane == 0) s_count[warp] = mine;
-            if (tail && mine_tail != 0) {
-                uint32_t at = 0;
-                if (lane == 0) at = atomicAdd(&s_pool_n, mine_tail);
-                at = __shfl_sync(kFull, at, 0);
-#pragma unroll
-                for (int r = 0; r < kR; ++r) {
-                    const uint32_t mine_at = at + (r == 1 ? __popc(to_tail[0]) : 0u) + __popc(to_tail[r] & lt);
-                    if (((to_tail[r] >> lane) & 1u) && mine_at < a.pool_len) pool[mine_at] = key[r];   // (an overflow is seen by the list warp)
-                }
-            }
             BlockSync();
             // ---- visited marks, while the list warp selects -------------------------------------------------------------------
             ++push;
@@ -426,55 +242,24 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                     }
                 }
             }
-            if (tail && s_cut != 0u) {
-                // scratch: the next push's place for new keys
-                uint32_t* free_words = reinterpret_cast<uint32_t*>(fkey + (push & 1u) * kFresh);
-                uint32_t bound;
-                const uint32_t kept = CutTail(pool, TailScratch{free_words, s_range, free_words + kTailBuckets + 4}, min(s_pool_n, a.pool_len), C - 32u * kList, false, &bound);
-                if (tid == 0) { s_pool_n = kept; s_tail_thr = bound; }
-                BlockSync();
-            }
         }
-        // ---- results: the ranks behind the list --------------------------------------------------------------------------------
         if (entry_pushes == 0) {
             for (uint32_t i = tid; i < C; i += kSlotThreads) a.out_cand[q * (uint64_t)C + i] = RecordOf(kNoKey);
             if (tid < 8) a.out_stats[q * 8 + tid] = tid == 5 ? 0xffffffffu : 0u;
-            return;
-        }
-        if (tail) {
-            BlockSync();   // the list warp's last merge
-            const uint32_t room = C - 32u * kList;
-            uint32_t n = min(s_pool_n, a.pool_len), fail = s_fail;
-            if (n != 0) {
-                uint32_t bound;
-                uint32_t* words32 = reinterpret_cast<uint32_t*>(fkey);
-                n = CutTail(pool, TailScratch{words32, s_range, words32 + kTailBuckets + 4}, n, room, true, &bound);
-                // copies of one node across the end of the list, in different states
-                if (n > room && (pool[room - 1] >> 2) == (pool[room] >> 2)) {
-                    uint32_t b = room, e = room;
-                    while (b > 0 && (pool[b - 1] >> 2) == (pool[room] >> 2)) --b;
-                    while (e < n && (pool[e] >> 2) == (pool[room] >> 2)) ++e;
-                    if (pool[b] != pool[e - 1]) fail = 1;   // ascending: the states differ exactly when first and last do
-                }
-            }
-            Cand* out = a.out_cand + q * (uint64_t)C + 32u * kList;
-            for (uint32_t i = tid; i < room; i += kSlotThreads) out[i] = RecordOf(i < n ? pool[i] : kNoKey);
-            if (tid == 0 && fail != 0u) a.out_stats[q * 8 + 6] = 1u;
         }
     } else {
         // ================================================ list warp =========================================================
-        const uint32_t L = a.p.top_l, cap = min(C, 32u * kList);   // ranks kept here
+        const uint32_t L = a.p.top_l;
         unsigned long long list[kList];
 #pragma unroll
         for (int r = 0; r < kList; ++r) list[r] = kNoKey;
         if (lane == 0) {
             s_thr = kNoKey;
-            s_pool_n = 0; s_tail_thr = 0xffffffffu; s_fail = 0; s_nsel = 0; s_cut = 0;
+            s_nsel = 0;
         }
-        uint32_t valid = 0, visited = 0, expanded = 0, iterations = 0, first_full = 0xffffffffu, hash_iter = 0, fail = 0;
-        // The first unexpanded entries of the list and their ranks: for W <= 2 the same in every lane, else lane x holds the
-        // x-th one (in un_key_0). And the keys of ranks L - 1 and L - 2: a new key below them lies within the first L ranks,
-        // alone or behind one other new key.
+        uint32_t valid = 0, visited = 0, expanded = 0, iterations = 0, first_full = 0xffffffffu, hash_iter = 0;
+        // The first two unexpanded entries of the list and their ranks, and the keys of ranks L - 1 and L - 2: a new key below
+        // them lies within the first L ranks, alone or behind one other new key.
         unsigned long long un_key_0 = kNoKey, un_key_1 = kNoKey, at_end_0 = kNoKey, at_end_1 = L > 1 ? kNoKey : 0ull;
         uint32_t un_pos_0 = 0, un_pos_1 = 0;
         constexpr uint32_t kSeg = 32u * kR;
@@ -490,7 +275,6 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 const uint32_t at = i + (i >= e2 ? 3u * kSeg - e2 : (i >= e1 ? 2u * kSeg - e1 : (i >= e0 ? kSeg - e0 : 0u)));
                 return i < n ? fresh[at] : kNoKey;
             };
-            const uint32_t pool_n = tail ? s_pool_n : 0u;
             const bool more = push + 1 < entry_pushes;   // the next push takes entries again
             // ---- selection -----------------------------------------------------------------------------------------------------
             const unsigned long long k0 = new_key(lane);
@@ -507,94 +291,39 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                     m0 = k < m0 ? k : m0;
                 }
                 const unsigned long long s0 = WarpMinKey(m0);
-                if (W <= 2) {
-                    const uint32_t holders = __ballot_sync(kFull, m0 == s0);
-                    const bool owner = m0 == s0 && (holders & ((1u << lane) - 1u)) == 0u;
-                    const unsigned long long s1 = WarpMinKey(owner ? m1 : m0);
-                    const bool new_first = s0 < un_key_0;
-                    if (new_first ? s0 < at_end_0 : un_key_0 < kNoKey) {
-                        nsel = 1;
-                        uint32_t id0, id1 = 0;
-                        if (new_first) { done_key = s0; done = 1; id0 = (uint32_t)s0 >> 2; }
-                        else { last_old = un_key_0; list_end = un_pos_0 + 1u; id0 = (uint32_t)last_old >> 2; }
-                        if (W == 2) {
-                            const unsigned long long s = new_first ? s1 : s0, u = new_first ? un_key_0 : un_key_1;
-                            const uint32_t u_pos = new_first ? un_pos_0 + 1u : un_pos_1;
-                            if (s < u) {
-                                if (s < (new_first ? at_end_1 : at_end_0)) {
-                                    nsel = 2;
-                                    id1 = (uint32_t)s >> 2;
-                                    done = s == done_key ? 2u : 1u;
-                                    done_key = s;
-                                }
-                            } else if (u < kNoKey && u_pos < L) {
+                const uint32_t holders = __ballot_sync(kFull, m0 == s0);
+                const bool owner = m0 == s0 && (holders & ((1u << lane) - 1u)) == 0u;
+                const unsigned long long s1 = WarpMinKey(owner ? m1 : m0);
+                const bool new_first = s0 < un_key_0;
+                if (new_first ? s0 < at_end_0 : un_key_0 < kNoKey) {
+                    nsel = 1;
+                    uint32_t id0, id1 = 0;
+                    if (new_first) { done_key = s0; done = 1; id0 = (uint32_t)s0 >> 2; }
+                    else { last_old = un_key_0; list_end = un_pos_0 + 1u; id0 = (uint32_t)last_old >> 2; }
+                    if (W == 2) {
+                        const unsigned long long s = new_first ? s1 : s0, u = new_first ? un_key_0 : un_key_1;
+                        const uint32_t u_pos = new_first ? un_pos_0 + 1u : un_pos_1;
+                        if (s < u) {
+                            if (s < (new_first ? at_end_1 : at_end_0)) {
                                 nsel = 2;
-                                id1 = (uint32_t)u >> 2;
-                                last_old = u;
-                                list_end = (new_first ? un_pos_0 : un_pos_1) + 1u;
+                                id1 = (uint32_t)s >> 2;
+                                done = s == done_key ? 2u : 1u;
+                                done_key = s;
                             }
-                        }
-                        if (lane < 2) s_node[lane] = lane == 0 ? id0 : id1;
-                    }
-                } else {
-                    // general widths, one selection after the other
-                    unsigned long long s_min = s0;
-                    uint32_t un_taken = 0, pick = 0, new_picks = 0;
-#pragma unroll 1
-                    while (nsel < W) {
-                        const unsigned long long u = __shfl_sync(kFull, un_key_0, un_taken);
-                        if (s_min < u) {
-                            uint32_t below = new_picks;
-#pragma unroll
-                            for (int r = 0; r < kList; ++r) below += __popc(__ballot_sync(kFull, list[r] < s_min));
-                            if (below >= L) break;
-                            if (lane == nsel) pick = (uint32_t)s_min >> 2;
-                            done = s_min == done_key ? done + 1u : 1u;
-                            done_key = s_min;
-                            ++nsel;
-                            ++new_picks;
-                            // the next one: another copy of the same key, or the least above it
-                            uint32_t copies = 0;
-                            unsigned long long least = kNoKey;
-#pragma unroll 1
-                            for (uint32_t i = 0; i < n; i += 32u) {
-                                const unsigned long long k = new_key(i + lane);
-                                copies += __popc(__ballot_sync(kFull, k == done_key));
-                                if (k > done_key && k < least) least = k;
-                            }
-                            s_min = copies > done ? done_key : WarpMinKey(least);
-                        } else if (u < kNoKey) {
-                            const uint32_t pos = __shfl_sync(kFull, un_pos_0, un_taken);
-                            if (pos + new_picks >= L) break;
-                            if (lane == nsel) pick = (uint32_t)u >> 2;
+                        } else if (u < kNoKey && u_pos < L) {
+                            nsel = 2;
+                            id1 = (uint32_t)u >> 2;
                             last_old = u;
-                            list_end = pos + 1u;
-                            ++un_taken;
-                            ++nsel;
-                        } else {
-                            break;
+                            list_end = (new_first ? un_pos_0 : un_pos_1) + 1u;
                         }
                     }
-                    if (lane < nsel) s_node[lane] = pick;
+                    if (lane < 2) s_node[lane] = lane == 0 ? id0 : id1;
                 }
             }
-            // the pool must take this push's displaced entries and the next push's tail keys
-            const bool cut = tail && pool_n + n + kFresh > a.pool_len;
-            if (lane == 0) {
-                s_nsel = nsel;
-                if (tail) s_cut = cut ? 1u : 0u;
-            }
+            if (lane == 0) s_nsel = nsel;
             BlockSync();   // the selection is there
             const bool last_push = !more && nsel == 0;
-            if (tail && pool_n > a.pool_len) fail = 1;
-            if (cut && !last_push) BlockSync();
             // ---- merge, behind the next push's loads ------------------------------------------------------------------------------
-            const uint32_t nv = (uint32_t)min((uint64_t)C, (uint64_t)valid + fv);
-            if (first_full == 0xffffffffu && nv >= L) first_full = push < entry_pushes ? 0u : iterations;
-            visited += fv;
-            valid = nv;
-            iterations += nsel != 0u ? 1u : 0u;
-            expanded += nsel;
             if (list_end != 0u) {   // every unexpanded entry up to there was selected; a twin of the last one stays behind it
 #pragma unroll
                 for (int r = 0; r < kList; ++r) {
@@ -602,6 +331,16 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                     else if (((list[r] ^ last_old) >> 2) == 0ull) list[r] = (list[r] & ~3ull) | kTwin;
                 }
             }
+            // The merge below takes 32 keys at a time. Where several such merges meet a full list that may hold copies of theirs (behind
+            // rank L), a later one must not displace an old copy that an earlier one left in its place: until the last of them
+            // new copies are kLate, behind the old ones, and so the first to drop out.
+            const bool late = n > 32u && C > L && valid != 0u && (uint64_t)valid + fv > C;
+            const uint32_t nv = (uint32_t)min((uint64_t)C, (uint64_t)valid + fv);
+            if (first_full == 0xffffffffu && nv >= L) first_full = push < entry_pushes ? 0u : iterations;
+            visited += fv;
+            valid = nv;
+            iterations += nsel != 0u ? 1u : 0u;
+            expanded += nsel;
             uint32_t copies = 0;
 #pragma unroll 1
             for (uint32_t c = 0; c < n; c += 32u) {
@@ -612,6 +351,7 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                     else if (k == done_key) k |= copies + __popc(same & ((1u << lane) - 1u)) < done ? kExpanded : kTwin;
                     copies += __popc(same);
                 }
+                if (late && ((uint32_t)k & 3u) == kNew) k |= kLate;
                 // descending order by rank counting
                 s_sort[lane] = k;
                 __syncwarp();
@@ -628,32 +368,17 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 __syncwarp();
                 s_sort[31u - rank] = k;
                 __syncwarp();
-                unsigned long long out = MergeIntoList<kList>(list, s_sort[lane], lane);
+                MergeIntoList<kList>(list, s_sort[lane], lane, late ? ~0ull : ~3ull);
                 __syncwarp();
-                if (tail) {
-                    const uint32_t b = __ballot_sync(kFull, out != kNoKey);
-                    if (b != 0u) {
-                        uint32_t at = 0;
-                        if (lane == 0) at = atomicAdd(&s_pool_n, (uint32_t)__popc(b));
-                        at = __shfl_sync(kFull, at, 0);
-                        if (at + (uint32_t)__popc(b) > a.pool_len) fail = 1;
-                        at += __popc(b & ((1u << lane) - 1u));
-                        if (out != kNoKey && at < a.pool_len) pool[at] = out;
-                    }
-                } else if (C > L) {
-                    // copies of one node across the end of the list, in different states
-                    const unsigned long long last = __shfl_sync(kFull, list[kList - 1], (cap - 1u) & 31u);
-                    if (__any_sync(kFull, out != kNoKey && ((out ^ last) >> 2) == 0ull && out != last)) fail = 1;
-                }
-                if (cap < 32u * kList) {   // a list shorter than the registers hold (kList is 1)
-                    const unsigned long long last = __shfl_sync(kFull, list[0], cap - 1u);
-                    const bool beyond = lane >= cap && list[0] != kNoKey;
-                    if (C > L && __any_sync(kFull, beyond && ((list[0] ^ last) >> 2) == 0ull && list[0] != last)) fail = 1;
-                    if (beyond) list[0] = kNoKey;
-                }
+            }
+            if (late) {
+#pragma unroll
+                for (int r = 0; r < kList; ++r)
+                    if (((uint32_t)list[r] & 3u) == kLate && list[r] != kNoKey) list[r] &= ~3ull;
+                SortCopies<kList>(list, lane);
             }
             if (last_push) break;
-            if (lane == ((cap - 1u) & 31u)) *reinterpret_cast<volatile unsigned long long*>(&s_thr) = list[kList - 1];
+            if (lane == 31u) *reinterpret_cast<volatile unsigned long long*>(&s_thr) = list[kList - 1];
             if (++hash_iter >= 3) {
                 hash_iter = 0;
 #pragma unroll
@@ -675,35 +400,24 @@ beam_short_kernel(const __grid_constant__ BeamArgs a) {
                 open += __popc(b);
             }
             __syncwarp();
-            if (W <= 2) {
-                un_key_0 = open > 0u ? s_open_key[0] : kNoKey;
-                un_pos_0 = s_open_rank[0];
-                un_key_1 = W == 2u && open > 1u ? s_open_key[1] : kNoKey;
-                un_pos_1 = s_open_rank[1];
-                at_end_0 = s_end[0];
-                if (L > 1u) at_end_1 = s_end[1];
-            } else {
-                un_key_0 = lane < open ? s_open_key[lane] : kNoKey;
-                un_pos_0 = s_open_rank[lane];
-            }
+            un_key_0 = open > 0u ? s_open_key[0] : kNoKey;
+            un_pos_0 = s_open_rank[0];
+            un_key_1 = W == 2u && open > 1u ? s_open_key[1] : kNoKey;
+            un_pos_1 = s_open_rank[1];
+            at_end_0 = s_end[0];
+            if (L > 1u) at_end_1 = s_end[1];
             __syncwarp();
         }
         if (entry_pushes == 0) return;
-        // ---- results: the list's ranks -----------------------------------------------------------------------------------------
+        // ---- results ------------------------------------------------------------------------------------------------------------
         Cand* out = a.out_cand + q * (uint64_t)C;
 #pragma unroll
-        for (int r = 0; r < kList; ++r)
-            if (r * 32u + lane < cap) out[r * 32u + lane] = RecordOf(list[r]);
+        for (int r = 0; r < kList; ++r) out[r * 32u + lane] = RecordOf(list[r]);
         if (lane == 0) {
             uint32_t* st = a.out_stats + q * 8;
             st[0] = visited; st[1] = expanded; st[2] = 0; st[3] = iterations;
-            st[4] = valid; st[5] = first_full; st[7] = 0;
-            st[6] = fail;   // the slot warps may set it once more, behind the next barrier
-            s_fail = fail;
-            __threadfence_block();
+            st[4] = valid; st[5] = first_full; st[6] = 0; st[7] = 0;
         }
-        if (tail) BlockSync();
-        for (uint32_t i = 32u * kList + lane; !tail && i < C; i += 32u) out[i] = RecordOf(kNoKey);
     }
 }
 

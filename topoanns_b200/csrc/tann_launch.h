@@ -21,11 +21,9 @@ struct FastPlan {
     int kind;             // 0 = codes, 1 = neighbour-code layout, 2 = node-id-range shards
     uint32_t rounds;      // slots per thread
     uint32_t list_regs;   // short form: list registers per lane; 0 = long form
-    uint32_t pool_len;    // short form: entries of the tail's pool
-    bool may_mark;        // short form: the long form is launched behind it for the queries it marks
     uint32_t list_len;
     bool two_lists, late;
-    uint32_t smem, long_smem;
+    uint32_t smem;
 };
 bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan);
 cudaError_t LaunchFast(BeamArgs a, const FastPlan& plan, uint64_t num_queries, cudaStream_t stream);
