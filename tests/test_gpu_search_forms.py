@@ -132,6 +132,32 @@ def _learned_stop(top_l):
     return ls
 
 
+# chunks of 1, 3, 4, 6 and 8 dims, and chunks of different widths (the last ones one dim wide)
+@pytest.mark.parametrize("chunks,dim", [(32, 32), (32, 96), (32, 128), (32, 100), (48, 48), (48, 144), (48, 101), (96, 96), (96, 576),
+                                        (96, 768), (96, 301)])
+@pytest.mark.parametrize("top_l,width,capacity", [(64, 2, 64), (40, 4, 64)])
+def test_table_built_in_the_kernel_gives_the_same_records_as_a_given_one(chunks, dim, top_l, width, capacity):
+    """The sums are the same operations in the same order: equal bits. width 4 on a degree of 64: the shared-memory list."""
+    degree = 64 if width == 4 else 32
+    ix, _, _, rng = _shared_neighbours(chunks, degree)
+    widths = np.full(chunks, dim // chunks)
+    if dim % chunks:
+        widths[:] = 1
+        widths[:chunks // 2] += rng.multinomial(dim - chunks, np.full(chunks // 2, 2.0 / chunks))
+    ix.dim = dim
+    ix.pq_chunk_offsets = torch.from_numpy(np.concatenate([[0], np.cumsum(widths)]).astype(np.int32)).cuda()
+    ix.pq_tables_col_major = torch.from_numpy(rng.normal(size=(dim, 256)).astype(np.float32)).cuda()
+    ix.pq_centroid = torch.from_numpy(rng.normal(size=dim).astype(np.float32)).cuda()
+    q = torch.from_numpy(rng.normal(size=(100, dim)).astype(np.float32)).cuda()
+    eo, ei = fixed_entries(100, [3, 700])
+    p = search.TopologySearchParams(top_k=1, top_l=top_l, search_width=width, max_expansions=512)
+    want, want_stats = search.beam_search(ix, p, eo, ei, lut=search.lut_build(ix, q), capacity=capacity)
+    got, got_stats = search.beam_search(ix, p, eo, ei, queries=q, capacity=capacity)
+    assert_candidates_equal(got, got_stats, np_u32(want), np_u32(want_stats))
+    general, general_stats = search.beam_search(_general_form(ix), p, eo, ei, queries=q, capacity=capacity)
+    assert_candidates_equal(got, got_stats, np_u32(general), np_u32(general_stats))
+
+
 # Distances that are NaN are not listed (no comparison with them holds), infinite ones are, by id. Where a list has them, the
 # count of valid entries runs ahead of the list.
 @pytest.mark.parametrize("chunks", [32, 48])

@@ -20,7 +20,6 @@ struct BeamArgs {
     uint32_t* status;
     // of beam_short_kernel and beam_long_kernel:
     uint32_t list_len, two_lists;   // long: entries of the list, whether it is double-buffered
-    const float* pivots_packed;  // PackPivots() of the index's pivots, or nullptr
 };
 
 }  // namespace tann

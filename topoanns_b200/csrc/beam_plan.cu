@@ -12,31 +12,6 @@ BeamKernelFn PickLong32(uint32_t rounds, int kind, bool late);
 BeamKernelFn PickLong48(uint32_t rounds, int kind, bool late);
 BeamKernelFn PickLong96(uint32_t rounds, int kind, bool late);
 
-// dims interleaved per pair of codes: [group of 32 (16) chunks][pair][chunk][dim of the chunk][code of the pair]
-__global__ void __launch_bounds__(256)
-pack_pivots_kernel(const float* __restrict__ col_major, uint32_t M, uint32_t sub, float* __restrict__ out) {
-    const uint64_t total = (uint64_t)M * sub * kCentroids;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t chunk_group = (uint32_t)(e / ((uint64_t)32 * sub * kCentroids));
-        const uint32_t width = min(32u, M - chunk_group * 32);
-        uint64_t r = e - (uint64_t)chunk_group * 32 * sub * kCentroids;
-        const uint32_t code_bit = (uint32_t)(r & 1u); r >>= 1;
-        const uint32_t dim = (uint32_t)(r % sub); r /= sub;
-        const uint32_t m = (uint32_t)(r % width); r /= width;
-        const uint32_t code = 2u * (uint32_t)r + code_bit;
-        out[e] = __ldg(col_major + (size_t)((chunk_group * 32 + m) * sub + dim) * kCentroids + code);
-    }
-}
-
-bool CanPackPivots(uint32_t M, uint32_t dim) {
-    return (M == 32 || M == 48 || M == 96) && (dim == 2 * M || dim == 4 * M || dim == 8 * M);
-}
-
-cudaError_t LaunchPackPivots(const float* col_major, uint32_t M, uint32_t dim, float* out, cudaStream_t stream) {
-    pack_pivots_kernel<<<SmCount() * 2, 256, 0, stream>>>(col_major, M, dim / M, out);
-    return cudaGetLastError();
-}
-
 static uint32_t ResidentBlocks(uint32_t smem) { return (228u * 1024u) / (smem + 1024u + 512u); }
 
 bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan) {

@@ -77,111 +77,109 @@ __device__ __forceinline__ float AdcXor(const unsigned char* lut, const uint32_t
 }
 
 // ---- the query's table, [code][chunk] per group of 32 (16) chunks --------------------------------------------------------
-// Packed pivots (PackPivots): per group, pair of codes and chunk the kSub dims of both codes interleaved, so that a lane
-// reads its chunk's values of two codes in one contiguous piece and the packed FP32 operations take them as they come.
-template <int kSub>
-__device__ __forceinline__ void PairEntries(const float* __restrict__ src, const float (&nq)[kSub], float2& acc) {
-    float t[2 * kSub];
+// Eight lanes read 128 consecutive bytes of a row of pivots (four codes each), and a lane does so for the rows of kPer chunks. The
+// table wants the chunks of a code side by side: writing chunk (step + lane) mod kPer at each step puts the 32 lanes on 32 banks,
+// for which a lane's kPer results are first rotated by its number (selects between registers, log2 kPer rounds).
+// What bounds it is the stream of dim KB of pivots per query out of L2. Whole calls of 2 k queries with top_l 64: 10 M x 128 uint8 390 ->
+// 327 us, 1 M x 768 float32 1176 -> 792 us against one row per lane (32 rows per request); against pivots that a launch in front laid
+// out anew 352 -> 352 and 921 -> 851 us.
+template <int kPer>
+__device__ __forceinline__ void RotateByLane(float4 (&v)[kPer], uint32_t by) {
 #pragma unroll
-    for (int i = 0; i < kSub / 2; ++i) *reinterpret_cast<float4*>(t + 4 * i) = __ldg(reinterpret_cast<const float4*>(src) + i);
-    acc = make_float2(0.0f, 0.0f);
+    for (int b = 1; b < kPer; b <<= 1) {
+        const bool on = (by & b) != 0;
+        float4 w[kPer];
 #pragma unroll
-    for (int s = 0; s < kSub; ++s) {
-        const float2 df = __fadd2_rn(make_float2(t[2 * s], t[2 * s + 1]), make_float2(nq[s], nq[s]));
-        acc = __ffma2_rn(df, df, acc);
+        for (int j = 0; j < kPer; ++j) {
+            const float4 x = v[j], y = v[(j + b) % kPer];
+            w[j] = make_float4(on ? y.x : x.x, on ? y.y : x.y, on ? y.z : x.z, on ? y.w : x.w);
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) v[j] = w[j];
     }
 }
-template <int kM, int kSub>
-__device__ __forceinline__ void TableFromPacked(float* lut, const float* sq, const float* __restrict__ packed, uint32_t tid) {
-    const uint32_t lane = tid & 31, warp = tid >> 5;
+__device__ __forceinline__ void AddSquares(float4& acc, const float4 v, float nq) {
+    const float2 n = make_float2(nq, nq);
+    const float2 a = __fadd2_rn(make_float2(v.x, v.y), n), b = __fadd2_rn(make_float2(v.z, v.w), n);
+    const float2 lo = __ffma2_rn(a, a, make_float2(acc.x, acc.y)), hi = __ffma2_rn(b, b, make_float2(acc.z, acc.w));
+    acc = make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+// The entries of a group of 4 * kPer chunks. sub: dims of every chunk (0: chunks of different widths).
+template <int kPer>
+__device__ __forceinline__ void GroupTable(float* lut, const float* sq, const BeamArgs& a, const float* given, uint32_t sub, uint32_t chunk0, uint32_t tid) {
+    const uint32_t p = tid & 7u, first = chunk0 + ((tid & 31u) >> 3) * kPer;
+    constexpr uint32_t width = kPer * 4;
+    float* t = lut + chunk0 * kCentroids + (first - chunk0);
+#pragma unroll 1
+    for (uint32_t c0 = (tid >> 5) * 32u + p * 4u; c0 < kCentroids; c0 += 128u) {
+        float4 acc[kPer];
 #pragma unroll
-    for (int g = 0; g * 32 < kM; ++g) {
-        const bool full = (g + 1) * 32 <= kM;
-        const uint32_t width = full ? 32u : 16u;
-        const uint32_t m = full ? lane : (lane & 15u), half = full ? 0u : lane >> 4;
-        float nq[kSub];
+        for (int j = 0; j < kPer; ++j) acc[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (given != nullptr) {
 #pragma unroll
-        for (int s = 0; s < kSub; ++s) nq[s] = -sq[(g * 32 + m) * kSub + s];
-        float* t = lut + g * 32 * kCentroids + m;
-        const float* src = packed + (size_t)g * 32 * kCentroids * kSub + m * kSub * 2;
-        // pairs of codes: warp, warp + 4, ... (both halves of a warp take a pair each in a group of 16 chunks)
-        const uint32_t pairs = full ? 128u : 64u;
-        constexpr int kAhead = kSub >= 8 ? 4 : (kSub >= 4 ? 8 : 16);
-        for (uint32_t p0 = warp; p0 < pairs; p0 += 4 * kAhead) {
-            float2 acc[kAhead];
+            for (int j = 0; j < kPer; ++j) acc[j] = __ldg(reinterpret_cast<const float4*>(given + (size_t)(first + j) * kCentroids + c0));
+        } else if (sub != 0) {
+            const float* rows = a.ix.pq_tables_col_major + (size_t)first * sub * kCentroids + c0;
+            const float* q = sq + first * sub;
+#pragma unroll 1
+            for (uint32_t s = 0; s < sub; ++s) {
+                float4 v[kPer];
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
-                const uint32_t cp = full ? p0 + 4 * u : 2 * (p0 + 4 * u) + half;
-                PairEntries<kSub>(src + (size_t)cp * width * kSub * 2, nq, acc[u]);
+                for (int j = 0; j < kPer; ++j) v[j] = __ldg(reinterpret_cast<const float4*>(rows + (size_t)(j * sub + s) * kCentroids));
+#pragma unroll
+                for (int j = 0; j < kPer; ++j) AddSquares(acc[j], v[j], -q[j * sub + s]);
             }
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < kPer; ++j) {
+                const uint32_t k1 = __ldg(a.ix.pq_chunk_offsets + first + j + 1);
+                float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+                for (uint32_t k = __ldg(a.ix.pq_chunk_offsets + first + j); k < k1; ++k)
+                    AddSquares(x, __ldg(reinterpret_cast<const float4*>(a.ix.pq_tables_col_major + (size_t)k * kCentroids + c0)), -sq[k]);
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
-                const uint32_t cp = full ? p0 + 4 * u : 2 * (p0 + 4 * u) + half;
-                // in a group of 16 the two halves write codes of different parity at a time: 32 banks
-                t[(2 * cp + half) * width] = half ? acc[u].y : acc[u].x;
-                t[(2 * cp + (half ^ 1u)) * width] = half ? acc[u].x : acc[u].y;
+                for (int u = 0; u < kPer; ++u)
+                    if (u == j) acc[u] = x;
             }
+        }
+        RotateByLane<kPer>(acc, p);
+#pragma unroll
+        for (int s = 0; s < kPer; ++s) {
+            const uint32_t m = (s + p) % kPer;
+            // rows of 16 chunks: lanes p and p + 4 write the same chunk, of codes of different parity
+            const bool odd = kPer == 4 && (p & 4u) != 0;
+            const float4 x = acc[s];
+            t[(c0 + (odd ? 1u : 0u)) * width + m] = odd ? x.y : x.x;
+            t[(c0 + (odd ? 0u : 1u)) * width + m] = odd ? x.x : x.y;
+            t[(c0 + (odd ? 3u : 2u)) * width + m] = odd ? x.w : x.z;
+            t[(c0 + (odd ? 2u : 3u)) * width + m] = odd ? x.z : x.w;
         }
     }
 }
-// The packed layout is for chunks of one width. Every warp checks all chunks, so that a block decides as one.
+// Dims of every chunk, or 0 when the chunks are of different widths. Every warp looks at all chunks, so that a block decides as one.
 template <int kM>
-__device__ __forceinline__ bool EqualChunks(const uint32_t* offsets, uint32_t dim, uint32_t lane) {
+__device__ __forceinline__ uint32_t EqualWidth(const uint32_t* offsets, uint32_t dim, uint32_t lane) {
     bool equal = dim % kM == 0;
 #pragma unroll
     for (uint32_t m = 0; m <= kM; m += 32)
         if (m + lane <= kM) equal = equal && __ldg(offsets + m + lane) == (m + lane) * (dim / kM);
-    return __all_sync(kFull, equal);
+    return __all_sync(kFull, equal) ? dim / kM : 0u;
 }
-// From the column-major pivots (any chunk widths), or copied from a caller's [M][256] table.
-template <int kM>
-__device__ __forceinline__ void TableFromColumns(float* lut, const float* sq, const BeamArgs& a, const float* given, uint32_t tid) {
-    const uint32_t lane = tid & 31, warp = tid >> 5;
-#pragma unroll 1
-    for (int g = 0; g * 32 < kM; ++g) {
-        const bool full = (g + 1) * 32 <= kM;
-        const uint32_t width = full ? 32u : 16u;
-        const uint32_t m = full ? lane : (lane & 15u), half = full ? 0u : lane >> 4;
-        const uint32_t chunk = g * 32 + m;
-        float* t = lut + g * 32 * kCentroids + m;
-        const uint32_t k0 = given ? 0u : __ldg(a.ix.pq_chunk_offsets + chunk), k1 = given ? 0u : __ldg(a.ix.pq_chunk_offsets + chunk + 1);
-        const uint32_t step = full ? 16u : 32u;
-#pragma unroll 4
-        for (uint32_t c0 = (full ? warp : 2 * warp + half) * 4; c0 < kCentroids; c0 += step) {
-            float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (given) {
-                acc = __ldg(reinterpret_cast<const float4*>(given + (size_t)chunk * kCentroids + c0));
-            } else {
-                for (uint32_t k = k0; k < k1; ++k) {
-                    const float4 v = __ldg(reinterpret_cast<const float4*>(a.ix.pq_tables_col_major + (size_t)k * kCentroids + c0));
-                    const float sv = sq[k];
-                    float df = v.x - sv; acc.x = fmaf(df, df, acc.x);
-                    df = v.y - sv; acc.y = fmaf(df, df, acc.y);
-                    df = v.z - sv; acc.z = fmaf(df, df, acc.z);
-                    df = v.w - sv; acc.w = fmaf(df, df, acc.w);
-                }
-            }
-            t[(c0 + 0) * width] = acc.x;
-            t[(c0 + 1) * width] = acc.y;
-            t[(c0 + 2) * width] = acc.z;
-            t[(c0 + 3) * width] = acc.w;
-        }
-    }
-}
-
-// Table of query q (tid: 0 to 127; sq: room for the query's values); `sync` is a barrier of these 128 threads.
+// Table of query q, built from the pivots or copied from the caller's [M][256] table (tid: 0 to 127; sq: room for the query's
+// values); `sync` is a barrier of these 128 threads.
 template <int kM, typename Sync>
 __device__ __forceinline__ void BuildTable(float* lut, float* sq, const BeamArgs& a, uint64_t q, uint32_t tid, Sync sync) {
     const uint32_t d = a.ix.dim;
     const float* given = a.lut != nullptr ? a.lut + q * (uint64_t)kM * kCentroids : nullptr;
-    const bool packed = a.pivots_packed != nullptr && EqualChunks<kM>(a.ix.pq_chunk_offsets, d, tid & 31);
-    if (given == nullptr)   // src/search/pq_query_tables.cu:33-52
+    uint32_t sub = 0;
+    if (given == nullptr) {   // src/search/pq_query_tables.cu:33-52
+        sub = EqualWidth<kM>(a.ix.pq_chunk_offsets, d, tid & 31);
         for (uint32_t i = tid; i < d; i += 128) sq[i] = LoadAsFloat<float>(a.queries, a.query_kind, q * d + i) - __ldg(a.ix.pq_centroid + i);
+    }
     sync();
-    if (packed && d == 2 * kM) TableFromPacked<kM, 2>(lut, sq, a.pivots_packed, tid);
-    else if (packed && d == 4 * kM) TableFromPacked<kM, 4>(lut, sq, a.pivots_packed, tid);
-    else if (packed && d == 8 * kM) TableFromPacked<kM, 8>(lut, sq, a.pivots_packed, tid);
-    else TableFromColumns<kM>(lut, sq, a, given, tid);
+#pragma unroll 1
+    for (uint32_t chunk0 = 0; chunk0 + 32 <= kM; chunk0 += 32) GroupTable<8>(lut, sq, a, given, sub, chunk0, tid);
+    if constexpr (kM % 32 != 0) GroupTable<4>(lut, sq, a, given, sub, kM / 32 * 32, tid);
     sync();
 }
 

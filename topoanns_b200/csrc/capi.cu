@@ -181,11 +181,11 @@ TannStatus tann_lut_build(const float* tables_col_major, const float* centroid,
     return TANN_OK;
 }
 
-// pivots_room: room for the index's pivots as LaunchPackPivots lays them out, or nullptr.
-static TannStatus BeamSearch(const TannIndexView* index, const TannBeamParams* params, const float* lut,
-                             float* pivots_room, const void* queries, uint32_t query_kind, uint64_t num_queries,
-                             const uint32_t* entry_offsets, const uint32_t* entry_ids, void* out_candidates,
-                             uint32_t* out_stats, uint32_t* status, tann_stream_t stream) {
+TannStatus tann_beam_search(const TannIndexView* index, const TannBeamParams* params, const float* lut,
+                            const void* queries, uint32_t query_kind, uint64_t num_queries,
+                            const uint32_t* entry_offsets, const uint32_t* entry_ids,
+                            void* out_candidates, uint32_t* out_stats, uint32_t* status,
+                            tann_stream_t stream) {
     TannStatus st = CheckBeam(index, params);
     if (st != TANN_OK) return st;
     if (num_queries == 0) return TANN_OK;
@@ -211,7 +211,7 @@ static TannStatus BeamSearch(const TannIndexView* index, const TannBeamParams* p
             if (st != TANN_OK) return st;
         }
     }
-    BeamPlan plan;
+    BeamPlan plan{};
     st = PlanBeam(index, params, num_queries, &plan);
     if (st != TANN_OK) return st;
     tann::BeamArgs a;
@@ -229,12 +229,6 @@ static TannStatus BeamSearch(const TannIndexView* index, const TannBeamParams* p
     a.out_stats = out_stats;
     a.status = status;
     if (plan.fast_form) {
-        // Laid out on each call (the caller may have changed the index's tables since the last one): 2.2 us for 128 x 256
-        // pivots, and one query's table takes 3 us from there against 22 us from the columns.
-        if (pivots_room != nullptr && lut == nullptr) {
-            TANN_CUDA(tann::LaunchPackPivots(index->pq_tables_col_major, index->num_chunks, index->dim, pivots_room, (cudaStream_t)stream));
-            a.pivots_packed = pivots_room;
-        }
         TANN_CUDA(tann::LaunchFast(a, plan.fast, num_queries, (cudaStream_t)stream));
         return TANN_OK;
     }
@@ -242,21 +236,12 @@ static TannStatus BeamSearch(const TannIndexView* index, const TannBeamParams* p
     return TANN_OK;
 }
 
-TannStatus tann_beam_search(const TannIndexView* index, const TannBeamParams* params, const float* lut,
-                            const void* queries, uint32_t query_kind, uint64_t num_queries,
-                            const uint32_t* entry_offsets, const uint32_t* entry_ids,
-                            void* out_candidates, uint32_t* out_stats, uint32_t* status,
-                            tann_stream_t stream) {
-    return BeamSearch(index, params, lut, nullptr, queries, query_kind, num_queries, entry_offsets, entry_ids,
-                      out_candidates, out_stats, status, stream);
-}
-
 TannStatus tann_beam_search_occupancy(const TannIndexView* index, const TannBeamParams* params,
                                       int lut_in_kernel, uint32_t* smem_bytes, uint32_t* blocks_per_sm,
                                       uint32_t* grid_blocks) {
     TannStatus st = CheckBeam(index, params);
     if (st != TANN_OK) return st;
-    BeamPlan plan;
+    BeamPlan plan{};
     (void)lut_in_kernel;
     st = PlanBeam(index, params, ~0ull, &plan);
     if (st != TANN_OK) return st;
@@ -702,7 +687,6 @@ struct TannSearcher {
     unsigned long long* d_counts;
     uint32_t* d_fixed_entries;   // max_entries ids: the fixed entry list before it is expanded per query
     uint32_t* d_status;          // TANN_STATUS_* bits of the last run
-    float* d_pivots;             // room for the PQ pivots laid out for the in-kernel table build (nullptr: other chunk shapes)
     uint32_t* h_status;
     // pinned staging
     // a batch that tann_searcher_submit enqueued and tann_searcher_wait has not collected yet
@@ -727,7 +711,6 @@ static void FreeSearcher(TannSearcher* s) {
     cudaFree(s->d_entry_ids); cudaFree(s->d_cand); cudaFree(s->d_cand_refined); cudaFree(s->d_stats);
     cudaFree(s->d_lut2); cudaFree(s->d_dists); cudaFree(s->d_ids); cudaFree(s->d_topk_dists);
     cudaFree(s->d_topk_ids); cudaFree(s->d_counts); cudaFree(s->d_fixed_entries); cudaFree(s->d_status);
-    cudaFree(s->d_pivots);
     cudaFreeHost(s->h_status);
     cudaFreeHost(s->h_queries); cudaFreeHost(s->h_topk_ids); cudaFreeHost(s->h_topk_dists);
     cudaFreeHost(s->h_stats); cudaFreeHost(s->h_entries);
@@ -772,7 +755,6 @@ TannStatus tann_searcher_create(const TannIndexView* index, uint64_t max_queries
     dev((void**)&s->d_counts, 16);
     dev((void**)&s->d_fixed_entries, (size_t)max_entries_per_query * 4);
     dev((void**)&s->d_status, 16);
-    if (tann::CanPackPivots(index->num_chunks, index->dim)) dev((void**)&s->d_pivots, d * 1024);
     host((void**)&s->h_status, 16);
     host(&s->h_queries, Q * d * 4);
     host((void**)&s->h_topk_ids, Q * max_top_n * 4);
@@ -867,8 +849,8 @@ TannStatus tann_searcher_run_device(TannSearcher* s, const TannBeamParams* beam,
         ei = s->d_entry_ids;
     }
     // traversal, table built in the kernel
-    TannStatus st = BeamSearch(&s->ix, beam, nullptr, s->d_pivots, queries_dev, query_kind, Q, eo, ei, s->d_cand,
-                               s->d_stats, s->d_status, stream);
+    TannStatus st = tann_beam_search(&s->ix, beam, nullptr, queries_dev, query_kind, Q, eo, ei, s->d_cand,
+                                     s->d_stats, s->d_status, stream);
     if (st != TANN_OK) return st;
     const void* cand = s->d_cand;
     uint32_t capacity = beam->candidate_capacity;

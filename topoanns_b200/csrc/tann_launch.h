@@ -28,9 +28,6 @@ struct FastPlan {
 bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan);
 cudaError_t LaunchFast(BeamArgs a, const FastPlan& plan, uint64_t num_queries, cudaStream_t stream);
 uint32_t FastBlocksPerSm(const FastPlan& plan);
-// The PQ pivots laid out for the in-kernel table build: dim * 256 floats.
-bool CanPackPivots(uint32_t M, uint32_t dim);
-cudaError_t LaunchPackPivots(const float* col_major, uint32_t M, uint32_t dim, float* out, cudaStream_t stream);
 
 cudaError_t LaunchLutBuild(const float* tables_col_major, const float* centroid,
                            const uint32_t* chunk_offsets, uint32_t dim, uint32_t M,
