@@ -451,9 +451,10 @@ typedef void (*BeamKernelFn)(const BeamArgs);
 template <int kM>
 BeamKernelFn PickLongOf(uint32_t rounds, int kind, bool late) {
     if (rounds == 1) {
-        if (kind == 2) return late ? nullptr : beam_long_kernel<kM, 1, 2, false>;
-        if (kind == 1) return late ? beam_long_kernel<kM, 1, 1, true> : beam_long_kernel<kM, 1, 1, false>;
-        return late ? beam_long_kernel<kM, 1, 0, true> : beam_long_kernel<kM, 1, 0, false>;
+        if (late) return kind == 2 ? nullptr : (kind == 1 ? beam_long_kernel<kM, 1, 1, true> : beam_long_kernel<kM, 1, 0, true>);
+        // (48 chunks: steps of up to 128 slots come here with the learned stop only)
+        if constexpr (kM != 48) return kind == 2 ? beam_long_kernel<kM, 1, 2, false> : (kind == 1 ? beam_long_kernel<kM, 1, 1, false> : beam_long_kernel<kM, 1, 0, false>);
+        return nullptr;
     }
     if (kind == 2) return late ? nullptr : beam_long_kernel<kM, 2, 2, false>;
     if (kind == 1) return late ? beam_long_kernel<kM, 2, 1, true> : beam_long_kernel<kM, 2, 1, false>;

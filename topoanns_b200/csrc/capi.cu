@@ -113,8 +113,8 @@ struct BeamPlan {
 
 TannStatus PlanBeam(const TannIndexView* ix, const TannBeamParams* p, uint64_t Q, BeamPlan* plan) {
     const uint32_t slots = p->search_width * ix->degree;
-    plan->fast_form = tann::PlanFast(*ix, *p, &plan->fast) && Q <= 0x7fffffffull;
-    if (Q == ~0ull) plan->fast_form = tann::PlanFast(*ix, *p, &plan->fast);
+    // (an occupancy query, Q == ~0, asks about batches of many waves)
+    plan->fast_form = tann::PlanFast(*ix, *p, Q == ~0ull ? 0x7fffffffull : Q, &plan->fast);
     if (plan->fast_form) {
         plan->smem = plan->fast.smem;
         plan->blocks_per_sm = (int)tann::FastBlocksPerSm(plan->fast);

@@ -25,7 +25,7 @@ struct FastPlan {
     bool two_lists, late;
     uint32_t smem;
 };
-bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, FastPlan* plan);
+bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, uint64_t num_queries, FastPlan* plan);
 cudaError_t LaunchFast(BeamArgs a, const FastPlan& plan, uint64_t num_queries, cudaStream_t stream);
 uint32_t FastBlocksPerSm(const FastPlan& plan);
 
