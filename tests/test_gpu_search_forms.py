@@ -201,3 +201,37 @@ def _not_finite(chunks, top_l, width, top_n, learned):
             w = np_u32(want)
             assert (w[1, :, 1] == 0xFFFFFFFF).all() and np_u32(want_stats)[1, 4] == min(cap, entries[1].numel() // 12)
             assert not np.isnan(w[:, :, 0].view(np.float32)).any()
+
+
+# on both sides of the batch sizes from which the pivots lie in shared memory (5 queries per SM up to 48 chunks, 20 up to 64)
+@pytest.mark.parametrize("chunks,dim,per_sm", [(16, 64, 5), (32, 64, 5), (48, 96, 5), (64, 128, 20), (96, 192, 20)])
+@pytest.mark.parametrize("top_l", [16, 100])
+def test_pq2_refine_at_the_lines_between_its_forms(chunks, dim, per_sm, top_l):
+    ix, _, codes, rng = _shared_neighbours(chunks, 32)
+    ix.dim = dim
+    ix.pq_chunk_offsets = torch.arange(0, dim + 1, dim // chunks, dtype=torch.int32, device="cuda")
+    normal = lambda *shape: torch.from_numpy(rng.normal(size=shape).astype(np.float32)).cuda()
+    ix.pq_tables_col_major, ix.pq_centroid = normal(dim, 256), normal(dim)
+    pages = search.device_index_from_arrays(adjacency=np.zeros((3000, 1), np.int32), codes=codes, vectors=rng.normal(size=(3000, dim)).astype(np.float32),
+                                            pq_tables_row_major=np.zeros((256, dim), np.float32), pq_centroid=np.zeros(dim, np.float32),
+                                            pq_chunk_offsets=np.arange(0, dim + 1, dim // chunks, dtype=np.uint32))
+    ix.vector_pages, ix.vector_bytes, ix.vectors_per_page = pages.vector_pages, pages.vector_bytes, pages.vectors_per_page
+    p2 = search.Pq2Resources(codes=torch.from_numpy(codes[::-1].copy()).cuda(), tables_col_major=normal(dim, 256), centroid=normal(dim),
+                             chunk_offsets=ix.pq_chunk_offsets, error_bounds=normal(3000).abs(), cross_terms=normal(chunks, 256, 256))
+    tp = search.TopologySearchParams(top_k=10, top_l=top_l, search_width=2, max_expansions=64)
+    rp = search.RerankExactParams(top_k=10, top_n=16, rank_tile_size=16, use_pq2_bound_filter=True)
+    line = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    for batch in (line - 1, line):
+        q = normal(batch, dim)
+        eo, ei = fixed_entries(batch, [7])
+        cand, stats = search.beam_search(ix, tp, eo, ei, queries=q, capacity=tp.capacity(16))
+        lut2 = search.lut_build(ix, q, tables_col_major=p2.tables_col_major, centroid=p2.centroid)
+        refined = search.pq2_refine(cand, stats, top_l, p2.codes, lut2, base_codes=ix.codes, cross_terms=p2.cross_terms)
+        d, i, _, _ = search.rerank_exact(ix, rp, refined, q, p2.error_bounds)
+        want_d, want_i = search.topk_pack(d, i, 10)
+        sr = search.Searcher(ix, batch, tp.capacity(16), 16, 1)
+        sr.set_pq2(p2, top_l)
+        got_i, got_d = sr.run_host(q.cpu().numpy(), tp, rp, np.array([7], np.uint32))[:2]
+        sr.close()
+        assert np.array_equal(got_i, np_u32(want_i))
+        assert np.array_equal(got_d.view(np.uint32), np_u32(want_d))

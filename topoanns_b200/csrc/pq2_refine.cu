@@ -260,14 +260,17 @@ cudaError_t LaunchPq2Refine(const void* cand, const uint32_t* stats, uint64_t Q,
     if (Q == 0 || refine_top_l == 0) return cudaSuccess;
     uint32_t padded = 1;
     while (padded < refine_top_l) padded <<= 1;
-    // The pivots take 98 KB at dim = 96; a batch has to be large enough to pay for loading them into every SM. M = 48, one
-    // block per query -> pivots in shared memory, for lists of 16 / 64 / 256: 148 queries 8.8 -> 11.9, 23.8 -> 26.0,
-    // 101.8 -> 85.9 us; 600 queries 14.5 -> 14.7, 34.9 -> 32.4, 108.5 -> 96.7; 10 k queries 115 -> 92, 340 -> 266,
-    // 1229 -> 900. The line is at four queries per SM.
+    // Loading the pivots (dim KB) into every SM has to pay, and more chunks mean more of the cross-term gathers that both forms have.
+    // One block per query / pivots in shared memory, lists of 16 / 64 / 256, speed of the second relative to the first:
+    //   M = 16 and 32 (dim 64 and 128): 592 queries 0.94-1.02 / 1.07-1.13 / 1.22-1.34, 700: 1.0-1.08 / 1.07-1.15 / 1.17-1.27, 10 k:
+    //   1.29-1.34 / 1.23-1.38 / 1.24-1.48; M = 48 (96): 592: 0.92 / 1.02 / 1.11, 700: 0.98 / 1.03 / 1.09, 1 500: 1.04 / 1.01 / 1.04,
+    //   10 k: 1.19 / 1.18 / 1.20 (112 -> 94, 325 -> 274, 1 153 -> 964 us); M = 64 (128): 592 to 1 500: 0.89-0.94 / 0.95 / 0.99-1.01,
+    //   3 000: 1.10 / 1.12 / 1.17; M = 96 (192): 0.60 to 0.83 at every size.
+    // Hence five queries per SM for up to 48 chunks, twenty for up to 64.
     const size_t shared = (size_t)dim * kCentroids * 4 + kPq2Groups * ((size_t)padded * 8 + (size_t)dim * 4);
-    if (lut2 == nullptr && selector_bits == nullptr && M <= 96 && Q >= (uint64_t)SmCount() * 4 && shared <= 227u * 1024u &&
+    if (lut2 == nullptr && selector_bits == nullptr && M <= 64 && Q >= (uint64_t)SmCount() * (M <= 48 ? 5 : 20) && shared <= 227u * 1024u &&
         (reinterpret_cast<uintptr_t>(t2_col_major) & 15u) == 0) {
-        const auto kernel = M <= 32 ? pq2_refine_shared_kernel<1> : (M <= 64 ? pq2_refine_shared_kernel<2> : pq2_refine_shared_kernel<3>);
+        const auto kernel = M <= 32 ? pq2_refine_shared_kernel<1> : pq2_refine_shared_kernel<2>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
         if (e != cudaSuccess) return e;
         kernel<<<(unsigned)SmCount(), kPq2Groups * kPq2GroupThreads, shared, stream>>>(
