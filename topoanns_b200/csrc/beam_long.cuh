@@ -1,5 +1,5 @@
-// Beam search for long lists (top_l up to 1024) and for the learned stop: chunk counts that are multiples of 16, at most 256
-// frontier slots per step, one query per 128-thread block, the list in shared memory. Table, early selection and records as
+// Beam search for steps of up to 256 frontier slots that the register list does not take (wider searches, lists of up to 1024 entries, the
+// learned stop): 32, 48 or 96 chunks, one query per 128-thread block, the list in shared memory. Table, early selection and records as
 // in beam_short.cuh; the merge is shared by the block: a new key's place is its rank among the new keys plus its lower bound
 // in the list, the taken places form a bitmap, and the entry of any other place p is old entry p - (taken places below p).
 // The same pass yields the bitmap of unexpanded ranks.
@@ -273,8 +273,7 @@ beam_long_kernel(const __grid_constant__ BeamArgs a) {
             }
             const uint32_t total = mv + n;
             while (n != 0) {   // once, unless a new key ties with the last entry of a full list
-                // Places of the new keys, one lane per key (warps 1 to 3; warp 0 selects the next nodes meanwhile): keys of
-                // this push below it, plus list entries below it.
+                // Places of the new keys, one lane per key (warps 1 to 3): keys of this push below it, plus list entries below it.
                 for (uint32_t c = warp - 1u; c * 32u < n && warp != 0; c += 3u) {
                     const uint32_t i = c * 32u + lane;
                     if (lane < 4u) fkey[n + lane] = kInvalidKey;   // the loop below takes four keys at a time

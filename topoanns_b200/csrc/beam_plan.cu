@@ -17,6 +17,7 @@ static uint32_t ResidentBlocks(uint32_t smem) { return (228u * 1024u) / (smem + 
 // Which form takes a call. Below: speed relative to the general form (beam_search.cu) on 100 k x 128 uint8 (degree 32), 10 M x 128 uint8
 // (degrees 32 and 64, with and without neighbour codes), 4 M x 96 float32 (64) and 1 M x 768 float32 (64), M = 32, 32, 48 and 96, batches
 // of 1 to 10 000.
+// Other chunk counts (16 and 64 have forms of their own there) stay with the general form: none of the configurations has them.
 // * Register list (widths 1 and 2; capacities C of 32, 64, 128 and 256, without the learned stop): 1.02 to 1.78 for C of up to 128. A
 //   list of 256 costs more per step, which a short search does not earn back: at width 2, C = 256 and L = 16 / 32 / 64 / 100
 //   M = 32 has 0.80-0.91 / 0.87-0.99 / 0.97-1.13 / 1.01-1.16, M = 96 0.77-0.79 / 0.82-0.88 / 0.92-1.03 / 0.98-1.11, at width 1 and
@@ -26,10 +27,11 @@ static uint32_t ResidentBlocks(uint32_t smem) { return (228u * 1024u) / (smem + 
 //   batch needs more than one wave. M = 32, C = 512, L = 400 / 512: 1.01-1.25 / 1.02-1.34 for 600 queries and more (0.85-1.0 for 150 and
 //   fewer; L of up to 128: 0.89-0.99; C = 1024, where as many blocks reside: 0.73-0.88); M = 96, C = 512 / 1024: 1.0-1.9 /
 //   1.46-1.8 from 150 queries on (one query: 0.79-1.0); with the learned stop M = 32, C = 512 1.0-1.2, M = 48, C up to 128 1.11-1.22
-//   for 2 k queries and more. Widths 3 and 4 lose (0.67-0.99 on a degree of 32). M = 96 with the learned stop and a list that ends
-//   at top_l: 1.0-1.15 at every batch size.
+//   for 2 k queries and more. Widths 3 and 4 lose (0.67-0.99 on a degree of 32), but for M = 96 (1.49-1.73). M = 96 with the learned
+//   stop and a list that ends at top_l: 1.0-1.15 at every batch size.
 // * Steps of 129 to 256 slots, which the general form takes in rounds through a sort in shared memory: the register list (degree 96,
-//   width 2: 1.5 to 7.1), for M = 96 at C = 256 and L below 64 and for all other calls the shared-memory list (1.2 to 6.5).
+//   width 2: 1.5 to 7.1), for M = 96 at C = 256 and L below 64 and for all other calls the shared-memory list (1.0 to 6.5; width 32
+//   on a degree of 8, which selects 32 nodes one by one, 0.94 to 1.1 for batches of up to 150).
 bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, uint64_t num_queries, FastPlan* plan) {
     *plan = FastPlan{};
     const uint32_t M = ix.num_chunks, C = p.candidate_capacity, L = p.top_l, W = p.search_width;
@@ -57,7 +59,7 @@ bool PlanFast(const TannIndexView& ix, const TannBeamParams& p, uint64_t num_que
     if (plan->rounds == 1) {
         const uint32_t general = (228u * 1024u) / ((uint32_t)BeamSmemBytes(M, C, 128u, L, ix.dim) + 1024u + 960u);
         const bool more_blocks = ResidentBlocks(plan->smem) > general && num_queries > (uint64_t)SmCount() * general;
-        const bool ahead = W <= 2 && ((more_blocks && (late || M == 96 || (M == 32 && L > 256))) || (M == 96 && late && C < 2 * L));
+        const bool ahead = (more_blocks && (M == 96 ? W <= 4 : W <= 2 && (late || (M == 32 && L > 256)))) || (M == 96 && W <= 2 && late && C < 2 * L);
         if (!ahead) return false;
     }
     return plan->smem <= 227u * 1024u - 512u;

@@ -1,5 +1,4 @@
-// The query's PQ table in shared memory and the sum of a code row over it, shared by the beam-search kernels for chunk counts
-// that are multiples of 16.
+// The query's PQ table in shared memory and the sum of a code row over it, shared by the beam-search kernels for 32, 48 and 96 chunks.
 //
 // The table lies as [code][chunk], 32 chunks = 32 banks. Lane l reads chunk c ^ l at step c, so the 32 lanes of a look-up
 // fall on 32 banks whatever their codes are (a table per chunk in a row of 256 entries: 2 to 3.5 wavefronts per look-up). The
