@@ -1083,7 +1083,8 @@ def main():
     pushes = float(stats[:, 3].mean()) + (128 + 2 * degree - 1) // (2 * degree)      # iterations + entry batches
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "frac_of_nominal_8tbs": achieved / 8000.0, "traffic": traffic, "peak_source": peak_src,
-                "kernel": "beam_search_kernel",
+                # (which form of the beam search serves a point depends on its sizes; the default point takes this one)
+                "kernel": "beam_search_kernel" if (L, cap) == (DEFAULT_POINT[0], 256) else "beam search",
                 "whole_step_gbs": (beam_bytes + rerank_bytes) * args.steps / (dev_ms * 1e-3) / 1e9}
     if round_trip_ns:
         # what the resident queries could move if a push cost exactly one dependent DRAM round trip
@@ -1117,7 +1118,7 @@ def main():
                 "h2d_bytes_per_step": q_host_bytes, "d2h_bytes_per_step": int(Q * 10 * 8),
                 "pipeline": f"{n_lanes} searchers on {n_lanes} streams, batches submitted in turn (copies of one overlap kernels of the others)",
                 "one_batch_at_a_time": total_q / (e2e_serial_ms * 1e-3)},
-        "gpu_launches": 6 * args.steps,  # rvq, pivot layout, beam, float->uint8 check, rerank, top-k pack (and the repeat of marked queries when the list is longer than top_l)
+        "gpu_launches": 5 * args.steps,  # rvq, beam, float->uint8 check, rerank, top-k pack
         "clocks": clocks,
         "roofline": roofline,
     }
