@@ -48,6 +48,27 @@ def test_beam_search_at_the_edges_of_the_list_widths(chunks, top_l, width, top_n
         assert_candidates_equal(cand, stats, want, want_stats)
 
 
+# on both sides of the batch sizes from which the shared-memory list takes steps of up to 128 slots: one wave of the general form,
+# per_sm blocks on an SM (0: at every size)
+@pytest.mark.parametrize("chunks,top_l,width,top_n,learned,per_sm", [(32, 400, 2, 64, False, 4), (32, 300, 1, 512, True, 4), (32, 64, 2, 512, True, 4),
+                                                                     (48, 64, 2, 64, True, 3), (48, 100, 1, 16, True, 3), (96, 100, 2, 300, False, 1),
+                                                                     (96, 600, 1, 64, True, 1), (96, 64, 2, 64, True, 0), (96, 200, 2, 64, True, 0)])
+def test_shared_memory_list_from_the_second_wave_on(chunks, top_l, width, top_n, learned, per_sm):
+    s, _ = _index(chunks)
+    ix = device_index(s)
+    line = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    p = search.TopologySearchParams(top_k=10, top_l=top_l, search_width=width, max_expansions=1024,
+                                    learned_stop=_learned_stop(top_l) if learned else None)
+    cap = p.capacity(top_n)
+    for batch in ((line, line + 1) if line else (33,)):
+        q = s.queries.cuda().float().repeat(batch // s.queries.shape[0] + 1, 1)[:batch].contiguous()
+        eo, ei = fixed_entries(batch, [s.medoid, 17, 400])
+        want, want_stats = search.beam_search(_general_form(ix), p, eo, ei, queries=q, capacity=cap)
+        for form in (ix, search.inline_neighbor_codes(dataclasses.replace(ix))):
+            got, got_stats = search.beam_search(form, p, eo, ei, queries=q, capacity=cap)
+            assert_candidates_equal(got, got_stats, np_u32(want), np_u32(want_stats))
+
+
 def _shared_neighbours(chunks, degree, nodes=3000, window=160, seed=5):
     """A graph in which parents share many neighbours, so that one push brings copies of a node and later ones bring it again; the
     codes are random, so that the copies end up anywhere in the list."""
