@@ -155,7 +155,7 @@ def _few_candidates(top_k, top_n=24):
 
 
 @pytest.mark.parametrize("top_k", [2, 7])
-def test_checker_moves_on_when_the_kth_distance_is_not_finite(top_k):
+def test_oracle_moves_on_when_the_kth_distance_is_not_finite(top_k):
     cand, q, pages, vpp, vb = _few_candidates(top_k)
     m = _stop([8, 12, 16], 4, {1: -4.0}, 1.0, -100.0, top_k=top_k)
     r = orc.rerank_learned(cand, q, pages, np.float32, model=m, top_n=24, top_k=top_k, tile=4, vectors_per_page=vpp,
